@@ -251,6 +251,12 @@ int unit_conv2d_plan_int8(const unit_conv_desc *desc, const void *d_x, const voi
                           const unit_epilogue *epilogue, void *d_out, void *d_workspace,
                           size_t workspace_bytes, unit_conv_plan *plan);
 int unit_conv2d_run(const unit_conv_plan *plan, void *stream);
+/* Points a plan at other buffers of the same shapes (the reference's built module is likewise called with
+ * new arrays each time): tile selection and tensor map stay, only addresses change.  d_x is the activations
+ * (or the A matrix), d_bias and d_residual are given exactly when the plan was made with them, d_workspace
+ * when the plan uses scratch.  Not to be called while another thread uses the same plan. */
+int unit_plan_rebind(unit_conv_plan *plan, const void *d_x, const int32_t *d_bias, const void *d_residual,
+                     void *d_out, void *d_workspace);
 
 /* Three-dimensional int8 convolution on NCDHW16c (replaces the compute of
  * apps/cpu/kernel/conv3d.py:58-64, scheduled by INTRINSICS['vnni'] like the two-dimensional one).
@@ -295,16 +301,23 @@ int unit_conv2d_u8s8_requant_nchwc_noalloc(const unit_conv_desc *desc, const uin
 int unit_dense_u8s8s32(int32_t m, int32_t n, int32_t k, const uint8_t *d_a, int64_t lda,
                        const void *d_packed_w, int32_t *d_c, int64_t ldc, void *stream);
 
+int unit_dense_plan_u8s8s32(int32_t m, int32_t n, int32_t k, const uint8_t *d_a, int64_t lda,
+                            const void *d_packed_w, int32_t *d_c, int64_t ldc, unit_conv_plan *plan);
+
 /* Replaces conv2d_NCHW16c_OHWI16o (python/tensorizer/ops/gpu.py:8-58).
  * d_x fp16 NCHW16c, d_out fp32 NCHW16c; desc->c_block must be 16. */
 int unit_conv2d_f16f32_nchw16c(const unit_conv_desc *desc, const void *d_x,
                                const void *d_packed_w, float *d_out, void *stream);
+int unit_conv2d_plan_f16f32(const unit_conv_desc *desc, const void *d_x, const void *d_packed_w,
+                            float *d_out, unit_conv_plan *plan);
 
 /* Replaces the tensor-core GEMM of apps/gpu/gemm.py:6-19 and
  * poc/tensorcore/gemm-prefetch.cu:66-164.  A fp16 [m][k] (row pitch lda
  * bytes), C fp32 [m][n] (row pitch ldc elements). */
 int unit_gemm_f16f32(int32_t m, int32_t n, int32_t k, const void *d_a, int64_t lda,
                      const void *d_packed_w, float *d_c, int64_t ldc, void *stream);
+int unit_gemm_plan_f16f32(int32_t m, int32_t n, int32_t k, const void *d_a, int64_t lda,
+                          const void *d_packed_w, float *d_c, int64_t ldc, unit_conv_plan *plan);
 
 /* ---- layout transforms --------------------------------------------------- */
 

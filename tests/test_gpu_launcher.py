@@ -1,0 +1,87 @@
+"""Repeated operator calls with packed weights run through the launcher (unit_b200/csrc/host_ext.cpp): a call
+of a geometry it has seen must read the buffers it is given, and calls it does not know must be checked as before."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope='module')
+def U():
+    import unit_b200
+    return unit_b200
+
+
+def gen(seed):
+    return torch.Generator(device='cuda').manual_seed(seed)
+
+
+def u8(shape, g):
+    return torch.randint(0, 256, shape, dtype=torch.uint8, device='cuda', generator=g)
+
+
+# operands described by a tensor map (re-addressed on each call), below its size limit (gathered), folded through
+# scratch, and the operators with float outputs
+CONV = [dict(x=(1, 4, 56, 56, 16), w=(4, 4, 3, 3, 4, 16, 4), stride=1, padding=1),
+        dict(x=(2, 4, 9, 9, 16), w=(4, 4, 3, 3, 4, 16, 4), stride=2, padding=(1, 1)),
+        dict(x=(3, 1, 64, 64, 4), w=(4, 1, 7, 7, 1, 16, 4), stride=2, padding=3)]
+
+
+@pytest.mark.parametrize('case', CONV)
+@pytest.mark.parametrize('form', ['raw', 'requant', 'residual'])
+def test_conv2d_calls_read_their_own_buffers(U, case, form):
+    g = gen(5)
+    w = torch.randint(-128, 128, case['w'], dtype=torch.int8, device='cuda', generator=g)
+    kw = dict(stride=case['stride'], padding=case['padding'])
+    pw = U.pack_conv_weights_int8(w, **kw)
+    for i in range(4):
+        x = u8(case['x'], g)
+        opt = dict(kw)
+        if form != 'raw':
+            opt.update(bias=torch.randint(-2 ** 12, 2 ** 12, (64,), dtype=torch.int32, device='cuda', generator=g),
+                       out_dtype='uint8', requant_shift=9)
+        if form == 'residual':
+            acc = U.conv2d_NCHWc_int8(x, pw, **kw)
+            opt['residual'] = u8(tuple(acc.shape), g)
+        got = U.conv2d_NCHWc_int8(x, pw, **opt)
+        want = U.conv2d_NCHWc_int8_plan(x, pw, **opt).run()     # planned anew for these buffers
+        named = torch.empty_like(got)
+        assert U.conv2d_NCHWc_int8(x, pw, out=named, **opt) is named
+        assert U.conv2d_NCHWc_int8(x, pw, out=named, **opt) is named
+        assert torch.equal(got, want) and torch.equal(named, want)
+        assert got.data_ptr() != x.data_ptr()
+    with torch.cuda.stream(torch.cuda.Stream()) as _:           # another stream waits for the weights first
+        torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+        for _ in range(2):
+            assert torch.equal(U.conv2d_NCHWc_int8(x, pw, **opt), want)
+    with pytest.raises(ValueError):
+        U.conv2d_NCHWc_int8(x[..., :4].contiguous() if x.shape[-1] == 16 else x.repeat(1, 1, 1, 1, 4), pw, **kw)
+    U.device_status()
+
+
+@pytest.mark.parametrize('m', [1, 70, 300])
+def test_products_and_fp16_convolutions_read_their_own_buffers(U, m):
+    g = gen(6)
+    wq = torch.randint(-128, 128, (4, 256, 16, 4), dtype=torch.int8, device='cuda', generator=g)
+    pd = U.pack_dense_weights_int8(wq)
+    dense = wq.permute(0, 2, 1, 3).reshape(64, 1024)
+    bf = torch.randn((512, 64), device='cuda', generator=g).half()
+    pg = U.pack_gemm_weights_f16(bf)
+    wf = torch.randn((2, 2, 3, 3, 16, 16), device='cuda', generator=g).half()
+    pf = U.pack_conv_weights_f16(wf)
+    wc = wf.permute(0, 5, 1, 4, 2, 3).reshape(32, 32, 3, 3).double()
+    for i in range(3):
+        a = u8((m, 1024), g)
+        assert np.array_equal(U.dense_dotprod(a, pd).cpu().numpy(), (a.cpu().to(torch.int64) @ dense.cpu().to(torch.int64).T).numpy())
+        ah = torch.randn((m, 512), device='cuda', generator=g).half()
+        # 512 products of fp16 values are exact in fp32; their fp32 sum is off by at most 512 * 2^-24 of the absolute sum
+        bound = 512 * 2.0 ** -24 * (ah.double().abs() @ bf.double().abs()) + 1e-30
+        assert bool(((U.gemm_f16f32(ah, pg).double() - ah.double() @ bf.double()).abs() <= bound).all())
+        x = torch.randn((m % 7 + 1, 2, 12, 12, 16), device='cuda', generator=g).half()
+        xc = x.permute(0, 1, 4, 2, 3).reshape(x.shape[0], 32, 12, 12).double()
+        got = U.conv2d_NCHW16c_OHWI16o(x, pf, 1, 1, padding=1).permute(0, 1, 4, 2, 3).reshape(x.shape[0], 32, 12, 12).double()
+        want = torch.nn.functional.conv2d(xc, wc, padding=1)
+        bound = 288 * 2.0 ** -24 * torch.nn.functional.conv2d(xc.abs(), wc.abs(), padding=1) + 1e-30
+        assert bool(((got - want).abs() <= bound).all())
+    U.device_status()

@@ -86,12 +86,16 @@ SIGNATURES = {
     'unit_conv2d_int8_nchwc': (_ci, [_dp, _vp, _vp, _ep, _vp, _vp, _sz, _vp]),
     'unit_conv2d_plan_int8': (_ci, [_dp, _vp, _vp, _ep, _vp, _vp, _sz, _pp]),
     'unit_conv2d_run': (_ci, [_pp, _vp]),
+    'unit_plan_rebind': (_ci, [_pp, _vp, _vp, _vp, _vp, _vp]),
     'unit_packed_weights_bytes_conv3d_i8': (_sz, [_d3]),
     'unit_pack_weights_conv3d_i8': (_ci, [_d3, _vp, _vp, _vp]),
     'unit_conv3d_int8_ncdhwc': (_ci, [_d3, _vp, _vp, _ep, _vp, _vp]),
     'unit_noalloc_scratch_capacity': (_sz, []),
     'unit_conv2d_u8s8_requant_nchwc_noalloc': (_ci, [_dp, _vp, _vp, _vp, _ci, _vp, _vp]),
     'unit_dense_u8s8s32': (_ci, [_ci, _ci, _ci, _vp, _i64, _vp, _vp, _i64, _vp]),
+    'unit_dense_plan_u8s8s32': (_ci, [_ci, _ci, _ci, _vp, _i64, _vp, _vp, _i64, _pp]),
+    'unit_conv2d_plan_f16f32': (_ci, [_dp, _vp, _vp, _vp, _pp]),
+    'unit_gemm_plan_f16f32': (_ci, [_ci, _ci, _ci, _vp, _i64, _vp, _vp, _i64, _pp]),
     'unit_conv2d_f16f32_nchw16c': (_ci, [_dp, _vp, _vp, _vp, _vp]),
     'unit_gemm_f16f32': (_ci, [_ci, _ci, _ci, _vp, _i64, _vp, _vp, _i64, _vp]),
     'unit_pack_data_nchw_to_nchwc': (_ci, [_vp, _vp, _ci, _ci, _ci, _ci, _ci, _ci, _vp]),
@@ -122,6 +126,28 @@ def lib() -> ctypes.CDLL:
         fn.argtypes = args
     _LIB = L
     return L
+
+
+_HOST = None
+
+
+def host():
+    """The CPython extension that runs repeated operator calls (``csrc/host_ext.cpp``), bound to the library."""
+    global _HOST
+    if _HOST is not None:
+        return _HOST
+    L = lib()
+    import torch  # noqa: F401  (the extension links against torch's libraries, which this import loads)
+    if not os.path.exists(_build.HOST_PATH):
+        raise ImportError(f'unit_b200: {_build.HOST_PATH} is missing; build it with `python -m unit_b200.build`.')
+    from . import _host
+    addr = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value  # noqa: E731
+    _host.bind(addr(L.unit_conv2d_run), addr(L.unit_plan_rebind), addr(L.unit_pack_data_nchw_to_nchwc),
+               addr(L.unit_unpack_data_nchwc_to_nchw))
+    from . import tile_table
+    _host.set_table_version(tile_table.version())
+    _HOST = _host
+    return _host
 
 
 class UnitError(RuntimeError):

@@ -1,15 +1,19 @@
-"""Builds ``libunit_b200.so`` in-tree with nvcc for sm_100a (no JIT cache)."""
+"""Builds ``libunit_b200.so`` (nvcc, sm_100a) and the CPython extension ``_host.so`` in-tree (no JIT cache)."""
 from __future__ import annotations
 
 import os
 import shutil
 import subprocess
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, 'libunit_b200.so')
 _SOURCES = [os.path.join(_HERE, 'csrc', 'unit_abi.cu')]
 _DEPS = _SOURCES + [os.path.join(_HERE, 'csrc', 'igemm_sm100.cuh'), os.path.join(_HERE, 'csrc', 'tensor_peak.cuh'),
                     os.path.join(os.path.dirname(_HERE), 'include', 'unit_b200.h')]
+HOST_PATH = os.path.join(_HERE, '_host.so')
+_HOST_SOURCE = os.path.join(_HERE, 'csrc', 'host_ext.cpp')
+_HOST_DEPS = [_HOST_SOURCE, os.path.join(os.path.dirname(_HERE), 'include', 'unit_b200.h')]
 
 
 def _nvcc() -> str:
@@ -19,14 +23,35 @@ def _nvcc() -> str:
     raise RuntimeError('nvcc not found: unit_b200 needs the CUDA toolkit to build its kernels')
 
 
-def is_fresh() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _newer(target: str, deps) -> bool:
+    if not os.path.exists(target):
         return False
-    t = os.path.getmtime(LIB_PATH)
-    return all(os.path.getmtime(s) <= t for s in _DEPS)
+    t = os.path.getmtime(target)
+    return all(os.path.getmtime(s) <= t for s in deps)
+
+
+def is_fresh() -> bool:
+    return _newer(LIB_PATH, _DEPS)
+
+
+def build_host(force: bool = False) -> str:
+    """The extension sees torch's tensors directly, so it is built against the installed torch."""
+    if _newer(HOST_PATH, _HOST_DEPS) and not force:
+        return HOST_PATH
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [shutil.which('g++') or 'g++', '-O2', '-std=c++17', '-shared', '-fPIC', '-fvisibility=hidden',
+           f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', '-o', HOST_PATH, _HOST_SOURCE]
+    cmd += ['-isystem', os.path.join(root, 'include'), '-isystem', os.path.join(root, 'include', 'torch', 'csrc', 'api', 'include'),
+            '-isystem', os.path.join(cuda, 'include'), '-I', sysconfig.get_paths()['include']]
+    cmd += ['-L', os.path.join(root, 'lib'), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch_python']
+    subprocess.run(cmd, check=True)
+    return HOST_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_host(force)
     if is_fresh() and not force:
         return LIB_PATH
     cmd = [_nvcc(), '-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',

@@ -758,6 +758,7 @@ struct PlanImpl {
   int32_t fold_n, fold_h2, fold_w2;  // fold_n > 0: the stem's 2 x 2 fold into scratch runs first
   const void *fold_src;
   void *fold_dst;
+  int32_t map_base;                  // what the tensor map's base address is: 0 = no map, 1 = the activations, 2 = fold_dst
   const void *kernel;
   IgemmParams p;
   unsigned char map[sizeof(CUtensorMap)];
@@ -891,6 +892,7 @@ static unsigned int *error_word_address() {
 template <int AMODE, int EPI, bool F16, int MAX_MT = 2>
 static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = nullptr) {
   IgemmParams &p = pl.p;
+  pl.map_base = tmap_in == nullptr ? 0 : (pl.fold_n > 0 ? 2 : 1);
   if (tmap_in) memcpy(pl.map, tmap_in, sizeof(CUtensorMap));
   else memset(pl.map, 0, sizeof(pl.map));
   p.bn = c.bn;
@@ -1018,6 +1020,15 @@ static FastDiv make_fast_div(uint32_t d) {
 // size take the cp.async gather instead, which loses nothing on problems that small.
 static bool tensor_map_allowed(long long tensor_bytes) { return tensor_bytes >= 131072; }
 
+// A driver entry point by name; nullptr where the driver has none.
+template <typename Fn>
+static Fn driver_fn(const char *name) {
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) fn = nullptr;
+  return reinterpret_cast<Fn>(fn);
+}
+
 // im2col-mode tensor map over NCHW16c activations, seen as the 5-D tensor
 //   (c = 16 channels of a chunk, w, h, d = image, n = channel chunk)
 // so that one copy walks kTileM consecutive output positions (w, then h, then image) of one
@@ -1027,14 +1038,7 @@ static bool make_im2col_map(CUtensorMap *map, const unit_conv_desc *d, const voi
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const int *, const int *, cuuint32_t, cuuint32_t, const cuuint32_t *,
                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeIm2col");
   if (!encode) return false;
   if (!tensor_map_allowed((long long)d->n * d->c_in * d->h * d->w * (f16 ? 2 : 1))) return false;
   if (d->c_block != 16 || d->pad_w > 15 || d->pad_h > 15 || d->kw > 16 || d->kh > 16 || d->stride_w > 8 || d->stride_h > 8)
@@ -1060,14 +1064,7 @@ static bool make_im2col_map_3d(CUtensorMap *map, const unit_conv3d_desc *d, cons
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const int *, const int *, cuuint32_t, cuuint32_t, const cuuint32_t *,
                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeIm2col");
   if (!encode) return false;
   if (!tensor_map_allowed((long long)d->c_in * d->d * d->h * d->w)) return false;
   if (d->pad_w > 15 || d->pad_h > 15 || d->pad_d > 15 || d->kw > 16 || d->kh > 16 || d->kd > 16 || d->stride_w > 8 ||
@@ -1125,14 +1122,7 @@ static bool make_box_map(CUtensorMap *map, int n, int c_in, int h, int w, const 
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
   if (!encode || !tensor_map_allowed((long long)(depth > 0 ? depth : n) * c_in * h * w)) return false;
   const cuuint64_t cc = (cuuint64_t)c_in / 16;
   const cuuint64_t dims[4] = {(cuuint64_t)w * 2, (cuuint64_t)h, cc, (cuuint64_t)(depth > 0 ? depth : n)};
@@ -1154,14 +1144,7 @@ static bool make_dense_map(CUtensorMap *map, const void *a, long long rows, long
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
   if (!encode || ld >= (1ll << 40) || rows > 0x7fffffffll - 512) return false;
   if (!tensor_map_allowed((rows - 1) * ld + row_bytes)) return false;
   const cuuint64_t dims[3] = {2, (cuuint64_t)(row_bytes / 16), (cuuint64_t)rows};
@@ -1182,14 +1165,7 @@ static bool make_box_map_f16(CUtensorMap *map, int n, int c_in, int h, int w, co
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
   if (!encode || !tensor_map_allowed(2ll * n * c_in * h * w)) return false;
   const cuuint64_t cc = (cuuint64_t)c_in / 16;
   const cuuint64_t dims[5] = {4, (cuuint64_t)w, (cuuint64_t)h, cc, (cuuint64_t)n};
@@ -1210,14 +1186,7 @@ static bool make_pair_map(CUtensorMap *map, int n, int c_in, int h, int w, const
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
   if (!encode || (w & 1) || !tensor_map_allowed((long long)n * c_in * h * w)) return false;
   if (2 * g.bh - 1 > 256) return false;
   const cuuint64_t cc = (cuuint64_t)c_in / 16;
@@ -1240,14 +1209,7 @@ static bool make_dense_map_sw128(CUtensorMap *map, const void *a, long long rows
   typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-  static EncodeFn encode = [] {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      fn = nullptr;
-    return reinterpret_cast<EncodeFn>(fn);
-  }();
+  static const EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
   if (!encode || ld >= (1ll << 40) || rows > 0x7fffffffll - 512 || row_bytes >= (1ll << 31)) return false;
   if (!tensor_map_allowed((rows - 1) * ld + row_bytes)) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
@@ -1795,6 +1757,14 @@ int unit_conv2d_int8_nchwc(const unit_conv_desc *d, const void *x, const void *p
   return conv_i8(d, x, pw, e, out, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
+// Hands a filled plan to the caller's plain bytes.
+static int export_plan(int rc, const PlanImpl &pl, unit_conv_plan *plan) {
+  if (rc) return rc;
+  memset(plan, 0, sizeof(*plan));
+  memcpy(plan, &pl, sizeof(pl));
+  return UNIT_OK;
+}
+
 int unit_conv2d_plan_int8(const unit_conv_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out,
                           void *workspace, size_t workspace_bytes, unit_conv_plan *plan) {
   if (!plan) return UNIT_ERR_NULL;
@@ -1802,10 +1772,44 @@ int unit_conv2d_plan_int8(const unit_conv_desc *d, const void *x, const void *pw
   int rc = epilogue_from(epi, &e);
   if (rc) return rc;
   PlanImpl pl;
-  rc = plan_conv_i8(pl, d, x, pw, e, out, workspace, workspace_bytes);
-  if (rc) return rc;
-  memset(plan, 0, sizeof(*plan));
-  memcpy(plan, &pl, sizeof(pl));
+  return export_plan(plan_conv_i8(pl, d, x, pw, e, out, workspace, workspace_bytes), pl, plan);
+}
+
+int unit_plan_rebind(unit_conv_plan *plan, const void *x, const int32_t *bias, const void *residual, void *out, void *workspace) {
+  if (!plan || !x || !out) return UNIT_ERR_NULL;
+  PlanImpl *pl = reinterpret_cast<PlanImpl *>(plan);   // (8-byte aligned plain data in both forms)
+  if (pl->magic != kPlanMagic) return UNIT_ERR_SHAPE;
+  if (!aligned16(x) || !aligned16(out) || (bias && !aligned16(bias)) || (residual && !aligned16(residual)) ||
+      (workspace && !aligned16(workspace)))
+    return UNIT_ERR_ALIGN;
+  IgemmParams &p = pl->p;
+  // what the plan was made with or without stays so: the kernel variant and the bias step depend on it
+  if ((p.bias != nullptr) != (bias != nullptr) || (p.residual != nullptr) != (residual != nullptr)) return UNIT_ERR_SHAPE;
+  const void *base = nullptr, *old_base = nullptr;
+  if (pl->fold_n > 0) {
+    if (!workspace) return UNIT_ERR_NULL;
+    base = workspace;
+    old_base = pl->fold_dst;
+    pl->fold_src = x;
+    pl->fold_dst = workspace;
+  } else {
+    base = x;
+    old_base = p.a;
+  }
+  p.a = static_cast<const uint8_t *>(base);
+  p.bias = bias;
+  p.residual = static_cast<const uint8_t *>(residual);
+  p.out = out;
+  if (pl->map_base != 0 && base != old_base) {
+    alignas(64) CUtensorMap map;
+    memcpy(&map, pl->map, sizeof(map));
+    static const auto replace = driver_fn<CUresult (*)(CUtensorMap *, void *)>("cuTensorMapReplaceAddress");
+    if (!replace || replace(&map, const_cast<void *>(base)) != CUDA_SUCCESS) {
+      pl->magic = 0;   // half rebound: unusable
+      return UNIT_ERR_LAUNCH;
+    }
+    memcpy(pl->map, &map, sizeof(map));
+  }
   return UNIT_OK;
 }
 
@@ -1887,8 +1891,8 @@ int unit_conv2d_u8s8_requant_nchwc_noalloc(const unit_conv_desc *d, const uint8_
   return conv_i8(d, x, pw, e, out, scratch, need ? kStaticScratchBytes : 0, static_cast<cudaStream_t>(stream));
 }
 
-static int run_dense(bool f16, int32_t m, int32_t n, int32_t k, const void *a, int64_t lda, const void *pw, void *cmat,
-                     int64_t ldc, cudaStream_t st) {
+static int plan_dense(PlanImpl &pl, bool f16, int32_t m, int32_t n, int32_t k, const void *a, int64_t lda, const void *pw,
+                      void *cmat, int64_t ldc) {
   const int eb = f16 ? 2 : 1;
   const int kq = 16 / eb;  // elements per 16-byte K column
   if (m < 1 || n < 16 || n % 16 || k < kq || k % kq) return UNIT_ERR_SHAPE;
@@ -1898,7 +1902,7 @@ static int run_dense(bool f16, int32_t m, int32_t n, int32_t k, const void *a, i
   int rc = check_arch();
   if (rc) return rc;
   const TileCfg c = make_cfg(n, k / kq, false, true);
-  PlanImpl pl{};
+  pl = PlanImpl{};
   IgemmParams &p = pl.p;
   p.a = static_cast<const uint8_t *>(a); p.b = static_cast<const uint8_t *>(pw); p.out = cmat;
   p.m_total = m; p.n_total = n; p.lda = lda; p.ldc = ldc;
@@ -1913,7 +1917,28 @@ static int run_dense(bool f16, int32_t m, int32_t n, int32_t k, const void *a, i
     // matrices below the tensor-map size limit: the cp.async gather, single sub-tiles
     rc = f16 ? prepare<A_DENSE, EPI_RAW_ROWS, true, 1>(pl, c) : prepare<A_DENSE, EPI_RAW_ROWS, false, 1>(pl, c);
   }
+  return rc;
+}
+
+static int run_dense(bool f16, int32_t m, int32_t n, int32_t k, const void *a, int64_t lda, const void *pw, void *cmat,
+                     int64_t ldc, cudaStream_t st) {
+  PlanImpl pl;
+  const int rc = plan_dense(pl, f16, m, n, k, a, lda, pw, cmat, ldc);
   return rc ? rc : run_plan(pl, st);
+}
+
+int unit_dense_plan_u8s8s32(int32_t m, int32_t n, int32_t k, const uint8_t *a, int64_t lda, const void *pw, int32_t *cmat,
+                            int64_t ldc, unit_conv_plan *plan) {
+  if (!plan) return UNIT_ERR_NULL;
+  PlanImpl pl;
+  return export_plan(plan_dense(pl, false, m, n, k, a, lda, pw, cmat, ldc), pl, plan);
+}
+
+int unit_gemm_plan_f16f32(int32_t m, int32_t n, int32_t k, const void *a, int64_t lda, const void *pw, float *cmat, int64_t ldc,
+                          unit_conv_plan *plan) {
+  if (!plan) return UNIT_ERR_NULL;
+  PlanImpl pl;
+  return export_plan(plan_dense(pl, true, m, n, k, a, lda, pw, cmat, ldc), pl, plan);
 }
 
 int unit_dense_u8s8s32(int32_t m, int32_t n, int32_t k, const uint8_t *a, int64_t lda, const void *pw, int32_t *cmat,
@@ -1921,14 +1946,14 @@ int unit_dense_u8s8s32(int32_t m, int32_t n, int32_t k, const uint8_t *a, int64_
   return run_dense(false, m, n, k, a, lda, pw, cmat, ldc, static_cast<cudaStream_t>(stream));
 }
 
-int unit_conv2d_f16f32_nchw16c(const unit_conv_desc *d, const void *x, const void *pw, float *out, void *stream) {
+static int plan_conv_f16(PlanImpl &pl, const unit_conv_desc *d, const void *x, const void *pw, float *out) {
   int rc = check_conv(d, true);
   if (rc) return rc;
   if (!x || !pw || !out) return UNIT_ERR_NULL;
   if (!aligned16(x) || !aligned16(pw) || !aligned16(out)) return UNIT_ERR_ALIGN;
   if ((rc = check_arch())) return rc;
   const TileCfg c = make_cfg(d->c_out, conv_cols_f16(d), false);
-  PlanImpl pl{};
+  pl = PlanImpl{};
   IgemmParams &p = pl.p;
   p.a = static_cast<const uint8_t *>(x); p.b = static_cast<const uint8_t *>(pw); p.out = out;
   fill_conv(p, d, 2);
@@ -1947,7 +1972,19 @@ int unit_conv2d_f16f32_nchw16c(const unit_conv_desc *d, const void *x, const voi
     if (use_tma() && make_im2col_map(&map, d, x, true)) rc = prepare<A_CONV_TMA, EPI_RAW_NCHWC, true>(pl, c, &map);
     else rc = prepare<A_CONV_F16, EPI_RAW_NCHWC, true>(pl, c);
   }
+  return rc;
+}
+
+int unit_conv2d_f16f32_nchw16c(const unit_conv_desc *d, const void *x, const void *pw, float *out, void *stream) {
+  PlanImpl pl;
+  const int rc = plan_conv_f16(pl, d, x, pw, out);
   return rc ? rc : run_plan(pl, static_cast<cudaStream_t>(stream));
+}
+
+int unit_conv2d_plan_f16f32(const unit_conv_desc *d, const void *x, const void *pw, float *out, unit_conv_plan *plan) {
+  if (!plan) return UNIT_ERR_NULL;
+  PlanImpl pl;
+  return export_plan(plan_conv_f16(pl, d, x, pw, out), pl, plan);
 }
 
 int unit_gemm_f16f32(int32_t m, int32_t n, int32_t k, const void *a, int64_t lda, const void *pw, float *cmat,

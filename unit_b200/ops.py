@@ -54,11 +54,15 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+# operator numbers of the launcher (csrc/host_ext.cpp)
+_CONV2D, _CONV3D, _DENSE, _GEMM, _CONV_F16 = 1, 2, 3, 4, 5
+
 _TABLE_LOADED = False
+_HOST = None   # the bound extension, once a CUDA device and the library have been seen
 
 
 def _require_cuda_lib():
-    global _TABLE_LOADED
+    global _TABLE_LOADED, _HOST
     if not torch.cuda.is_available():
         raise RuntimeError('unit_b200 operators need a CUDA device (sm_100a); there is no CPU fallback')
     L = _lib.lib()
@@ -66,6 +70,7 @@ def _require_cuda_lib():
         _TABLE_LOADED = True
         from . import tile_table
         tile_table.load_default_table()   # per-shape tile overrides found by unit_b200.tune, if the file exists
+        _HOST = _lib.host()
     return L
 
 
@@ -100,6 +105,10 @@ class PackedWeights:
         self._ready = torch.cuda.Event()
         self._ready.record()
         self._synced = {_stream()}
+        # calls of known geometry run through the launcher, without the Python checks (csrc/host_ext.cpp)
+        self._launcher = _lib.host().Launcher(buf.device.index)
+        self._launcher.add_stream(_stream())
+        self._call = self._launcher.call
 
     def sync_to_current_stream(self) -> None:
         """Make the current stream wait for the pack kernel, once per stream.  (Not while the stream
@@ -110,6 +119,11 @@ class PackedWeights:
             return
         torch.cuda.current_stream().wait_event(self._ready)
         self._synced.add(st)
+        self._launcher.add_stream(st)
+
+    def _keep(self, plan: _CPlan, result: torch.Tensor, ws: Optional[torch.Tensor], c_out: int, *call) -> None:
+        """Hands the launcher the plan just made for this call (``call``: the arguments ``_call`` was tried with)."""
+        self._launcher.add(ctypes.addressof(plan), result, 0 if ws is None else ws.data_ptr(), c_out, *call)
 
     @property
     def nbytes(self) -> int:
@@ -264,20 +278,26 @@ class ConvPlan:
 
     def __init__(self, plan: _CPlan, out: torch.Tensor, keep: tuple):
         self._plan = plan
-        self._ref = ctypes.byref(plan)
         self.out = out
         self._keep = keep
-        self._run = _lib.lib().unit_conv2d_run
+        self._run = _lib.host().Runner(ctypes.addressof(plan), out).run
 
     def run(self) -> torch.Tensor:
-        rc = self._run(self._ref, torch.cuda.current_stream().cuda_stream)
-        if rc:
-            check(rc, 'unit_conv2d_run')
-        return self.out
+        r = self._run()
+        if type(r) is int:
+            check(r, 'unit_conv2d_run')
+        return r
 
 
-_PLAN_CACHE: dict = {}      # prepared launches of conv2d_NCHWc_int8 calls that named their output buffer
-_PLAN_CACHE_MAX = 512
+class _NamedLaunches:
+    """The prepared launches of calls that named their output buffer: the launchers keep them, one per
+    set of buffers."""
+
+    def __len__(self) -> int:
+        return _lib.host().bound_count()
+
+
+_PLAN_CACHE = _NamedLaunches()
 
 
 def _conv_int8_prepare(data, kernel, stride, padding, dilation, out_layout, out_dtype, bias, requant_shift, mul,
@@ -359,39 +379,21 @@ def conv2d_NCHWc_int8(data: torch.Tensor, kernel, stride: IntPair = 1, padding: 
     ``layout`` is accepted for signature compatibility; the channel block is
     read from ``data``'s last dimension as the reference's compute does.
     """
-    # Repeated calls on the same device buffers (the caller passes ``out``) reuse the prepared launch:
-    # the checks, the tile selection and the tensor-map encoding are done once per distinct call.
-    key = None
-    if out is not None and data.is_cuda and isinstance(kernel, PackedWeights):
-        from . import tile_table
-        key = (data.data_ptr(), tuple(data.shape), data.dtype, kernel.buf.data_ptr(), kernel.key, stride, padding, dilation,
-               out_layout, out_dtype, None if bias is None else (bias.data_ptr(), bias.dtype, bias.numel()), requant_shift, mul,
-               None if residual is None else (residual.data_ptr(), tuple(residual.shape), residual.dtype),
-               out.data_ptr(), tuple(out.shape), out.dtype, out.is_contiguous(), _stream(), tile_table.version())
-        hit = _PLAN_CACHE.get(key)
-        if hit is not None:
-            rc = hit[1](hit[2], key[-2])
-            if rc:
-                check(rc, 'unit_conv2d_run')
-            return out
+    if type(kernel) is PackedWeights:
+        r = kernel._call(_CONV2D, data, bias, residual, out, stride, padding, dilation, out_layout, out_dtype, requant_shift, mul)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_conv2d_run')
     L, d, tensors, epi, out_t, ws, ws_bytes, host, n = _conv_int8_prepare(
         data, kernel, stride, padding, dilation, out_layout, out_dtype, bias, requant_shift, mul, residual, out)
-    if n == 0:
-        return out_t.cpu() if (host and out is None) else out_t
-    x, pw = tensors[0], tensors[1]
-    with torch.cuda.device(x.device):
-        if key is not None and tensors[2] is bias and tensors[3] is residual:
+    if n > 0:
+        x, pw = tensors[0], tensors[1]
+        with torch.cuda.device(x.device):
             plan = _CPlan()
             check(L.unit_conv2d_plan_int8(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
                                           ws_bytes, ctypes.byref(plan)), 'unit_conv2d_plan_int8')
-            if len(_PLAN_CACHE) >= _PLAN_CACHE_MAX:
-                _PLAN_CACHE.pop(next(iter(_PLAN_CACHE)))
-            # (the entry holds no tensor: like the call itself it is valid for as long as the caller's buffers are)
-            _PLAN_CACHE[key] = (plan, L.unit_conv2d_run, ctypes.byref(plan))
             check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
-        else:
-            check(L.unit_conv2d_int8_nchwc(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
-                                           ws_bytes, _stream()), 'unit_conv2d_int8_nchwc')
+            pw._keep(plan, out_t, ws, d.c_out, _CONV2D, data, bias, residual, out, stride, padding, dilation, out_layout, out_dtype,
+                     requant_shift, mul)
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -509,11 +511,15 @@ def conv3d_NCDHWc_int8(data: torch.Tensor, kernel, stride=1, padding=0, out_dtyp
 def dense_dotprod(data: torch.Tensor, weight, bias: Optional[torch.Tensor] = None, out_dtype: str = 'int32', *,
                   out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C[i][j] = sum_k u8 data[i][k] * s8 weight[j/T][k/4][j%T][k%4]  -> s32 [M][N]."""
-    L = _require_cuda_lib()
     if out_dtype != 'int32':
         raise ValueError("out_dtype must be 'int32'")
     if bias is not None:
         raise ValueError('bias is not supported (the reference passes None)')
+    if type(weight) is PackedWeights:
+        r = weight._call(_DENSE, data, None, None, out)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_conv2d_run')
+    L = _require_cuda_lib()
     host = not data.is_cuda
     data = _to_device(data, torch.uint8, 'data')
     if data.dim() != 2:
@@ -534,8 +540,11 @@ def dense_dotprod(data: torch.Tensor, weight, bias: Optional[torch.Tensor] = Non
             if tuple(out_t.shape) != (m, n) or out_t.dtype != torch.int32 or not out_t.is_cuda or not out_t.is_contiguous():
                 raise ValueError('out must be a contiguous CUDA int32 [M][N] tensor')
         if m > 0:
-            check(L.unit_dense_u8s8s32(m, n, k, _ptr(data), k, _ptr(pw.buf), _ptr(out_t), n, _stream()),
-                  'unit_dense_u8s8s32')
+            plan = _CPlan()
+            check(L.unit_dense_plan_u8s8s32(m, n, k, _ptr(data), k, _ptr(pw.buf), _ptr(out_t), n, ctypes.byref(plan)),
+                  'unit_dense_plan_u8s8s32')
+            check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
+            pw._keep(plan, out_t, None, n, _DENSE, data, None, None, out)
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -544,6 +553,10 @@ def dense_dotprod(data: torch.Tensor, weight, bias: Optional[torch.Tensor] = Non
 # --------------------------------------------------------------------------
 def pack_data_nchwc(x: torch.Tensor, c_block: int = 16) -> torch.Tensor:
     """NCHW -> ``[N][ceil(C/cb)][H][W][cb]`` on the device (python/tensorizer/ops/gpu.py:26-28)."""
+    if _HOST is not None:
+        r = _HOST.pack(x, c_block)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_pack_data_nchw_to_nchwc')
     L = _require_cuda_lib()
     if x.dim() != 4:
         raise ValueError('x must be NCHW')
@@ -561,6 +574,10 @@ def pack_data_nchwc(x: torch.Tensor, c_block: int = 16) -> torch.Tensor:
 
 def unpack_data_nchwc(x: torch.Tensor, channels: Optional[int] = None) -> torch.Tensor:
     """``[N][C/cb][H][W][cb]`` -> NCHW, keeping the first ``channels`` channels."""
+    if _HOST is not None:
+        r = _HOST.unpack(x, channels)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_unpack_data_nchwc_to_nchw')
     L = _require_cuda_lib()
     if x.dim() != 5:
         raise ValueError('x must be [N][C/cb][H][W][cb]')
@@ -613,9 +630,14 @@ def conv2d_NCHW16c_OHWI16o(a: torch.Tensor, b, stride_h: int = 1, stride_w: int 
     ``[N][O/16][OH][OW][16]`` fp32.  The reference convolves without padding;
     ``padding`` adds implicit zero padding.
     """
+    if type(b) is PackedWeights:
+        r = b._call(_CONV_F16, a, None, None, out, stride_h, stride_w, out_type, padding)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_conv2d_run')
     L = _require_cuda_lib()
     if out_type != 'float32':
         raise ValueError("out_type must be 'float32'")
+    call = (a, None, None, out, stride_h, stride_w, out_type, padding)
     padding = _pair(padding)
     host = not a.is_cuda
     a = _to_device(a, torch.float16, 'a')
@@ -649,8 +671,11 @@ def conv2d_NCHW16c_OHWI16o(a: torch.Tensor, b, stride_h: int = 1, stride_w: int 
                 raise ValueError(f'out must be a contiguous CUDA float32 tensor of shape {oshape}')
         if n == 0:
             return out_t.cpu() if (host and out is None) else out_t
-        check(L.unit_conv2d_f16f32_nchw16c(ctypes.byref(d), _ptr(a), _ptr(pw.buf), _ptr(out_t), _stream()),
-              'unit_conv2d_f16f32_nchw16c')
+        plan = _CPlan()
+        check(L.unit_conv2d_plan_f16f32(ctypes.byref(d), _ptr(a), _ptr(pw.buf), _ptr(out_t), ctypes.byref(plan)),
+              'unit_conv2d_plan_f16f32')
+        check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
+        pw._keep(plan, out_t, None, c_out, _CONV_F16, *call)
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -673,6 +698,10 @@ def conv2d_NCHW16c_OHWI16o_compute(attrs, inputs, out_type='float32'):
 
 def gemm_f16f32(a: torch.Tensor, b, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C[M][N] fp32 = A[M][K] fp16 . B[K][N] fp16 with fp32 accumulation."""
+    if type(b) is PackedWeights:
+        r = b._call(_GEMM, a, None, None, out)
+        if r is not None:
+            return r if type(r) is not int else check(r, 'unit_conv2d_run')
     L = _require_cuda_lib()
     host = not a.is_cuda
     a = _to_device(a, torch.float16, 'a')
@@ -694,8 +723,11 @@ def gemm_f16f32(a: torch.Tensor, b, *, out: Optional[torch.Tensor] = None) -> to
             if tuple(out_t.shape) != (m, n) or out_t.dtype != torch.float32 or not out_t.is_cuda or not out_t.is_contiguous():
                 raise ValueError('out must be a contiguous CUDA float32 [M][N] tensor')
         if m > 0:
-            check(L.unit_gemm_f16f32(m, n, k, _ptr(a), 2 * k, _ptr(pw.buf), _ptr(out_t), n, _stream()),
-                  'unit_gemm_f16f32')
+            plan = _CPlan()
+            check(L.unit_gemm_plan_f16f32(m, n, k, _ptr(a), 2 * k, _ptr(pw.buf), _ptr(out_t), n, ctypes.byref(plan)),
+                  'unit_gemm_plan_f16f32')
+            check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
+            pw._keep(plan, out_t, None, n, _GEMM, a, None, None, out)
     return out_t.cpu() if (host and out is None) else out_t
 
 

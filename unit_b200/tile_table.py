@@ -77,6 +77,8 @@ def set_table(entries: List[dict]) -> None:
             setattr(arr[i], f, int(e.get(f, 16 if f == 'c_block' else 0)))
     _lib.check(L.unit_tile_table_set(arr, len(entries)), 'unit_tile_table_set')
     _VERSION += 1
+    if _lib._HOST is not None:
+        _lib._HOST.set_table_version(_VERSION)
 
 
 def load_default_table() -> int:
