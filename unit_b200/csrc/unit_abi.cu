@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "igemm_sm100.cuh"
+#include "layout.cuh"
 #include "tensor_peak.cuh"
 
 namespace unit {
@@ -420,182 +421,8 @@ static int launch_pack(const PackParams &pp, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------
-// layout kernels (bandwidth work)
+// weight layout kernels (one-off)
 // ---------------------------------------------------------------------------
-// NCHW <-> [n][c/CB][hw][CB] as a register transpose of 4-byte words.  A thread owns one channel
-// block and the P = 4 / EB pixels of one 4-byte word: on the NCHW side it touches one word per
-// channel, and consecutive threads touch consecutive words of the same channel row (a warp reads
-// or writes 128 contiguous bytes per instruction); on the blocked side its P pixels x CB channels
-// are P * CB * EB contiguous bytes, moved as 16-byte vectors.  Needs h * w to be a multiple of P and
-// 16-byte aligned tensors; other shapes take the element loops below.
-template <int EB, int CB>
-__device__ __forceinline__ void transpose_words(const uint32_t (&in)[CB], uint32_t (&out)[CB]) {
-  // in[c] = P pixels of channel c;  out = pixel-major: P pixels x CB channels, EB bytes each
-  if constexpr (EB == 4) {
-#pragma unroll
-    for (int c = 0; c < CB; ++c) out[c] = in[c];
-  } else if constexpr (EB == 2) {
-#pragma unroll
-    for (int q = 0; q < CB / 2; ++q) {
-      out[q] = __byte_perm(in[2 * q], in[2 * q + 1], 0x5410);           // pixel 0: low halves
-      out[CB / 2 + q] = __byte_perm(in[2 * q], in[2 * q + 1], 0x7632);  // pixel 1: high halves
-    }
-  } else {
-#pragma unroll
-    for (int px = 0; px < 4; ++px)
-#pragma unroll
-      for (int q = 0; q < CB / 4; ++q) {
-        const uint32_t sel = (uint32_t)((4 + px) << 4 | px);
-        const uint32_t lo = __byte_perm(in[4 * q], in[4 * q + 1], sel);
-        const uint32_t hi = __byte_perm(in[4 * q + 2], in[4 * q + 3], sel);
-        out[px * (CB / 4) + q] = __byte_perm(lo, hi, 0x5410);
-      }
-  }
-}
-// the inverse: in = pixel-major words, out[c] = P pixels of channel c
-template <int EB, int CB>
-__device__ __forceinline__ void untranspose_words(const uint32_t (&in)[CB], uint32_t (&out)[CB]) {
-  if constexpr (EB == 4) {
-#pragma unroll
-    for (int c = 0; c < CB; ++c) out[c] = in[c];
-  } else if constexpr (EB == 2) {
-#pragma unroll
-    for (int q = 0; q < CB / 2; ++q) {
-      out[2 * q] = __byte_perm(in[q], in[CB / 2 + q], 0x5410);
-      out[2 * q + 1] = __byte_perm(in[q], in[CB / 2 + q], 0x7632);
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < CB / 4; ++q) {
-      // words of pixels 0..3 holding channels 4q .. 4q+3
-      const uint32_t p0 = in[q], p1 = in[CB / 4 + q], p2 = in[2 * (CB / 4) + q], p3 = in[3 * (CB / 4) + q];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t sel = (uint32_t)((4 + k) << 4 | k);
-        out[4 * q + k] = __byte_perm(__byte_perm(p0, p1, sel), __byte_perm(p2, p3, sel), 0x5410);
-      }
-    }
-  }
-}
-
-// With 16-channel blocks a thread's result is 64 bytes (four 16-byte pieces).  Written straight
-// from the thread, every store instruction of a warp would touch 32 separate half sectors; the
-// pieces go through shared memory instead, so that consecutive lanes store consecutive 16 bytes
-// (512 contiguous bytes per warp instruction).  kPackPad staggers the four piece planes by 32 bytes,
-// which makes both the writes and the reads of the staging buffer conflict-free.
-constexpr int kPackThreads = 256, kPackPad = 2;
-template <int EB, int CB>
-__global__ void __launch_bounds__(kPackThreads)
-    nchw_to_nchwc_vec_kernel(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, int n, int c, long long hw_words) {
-  constexpr int NP = CB / 4;  // 16-byte pieces per thread
-  __shared__ uint4 stage[NP > 1 ? NP * (kPackThreads + kPackPad) : 1];
-  const int cc = (c + CB - 1) / CB;
-  const long long total = (long long)n * cc * hw_words;
-  const long long span = (long long)gridDim.x * blockDim.x;
-  for (long long base = blockIdx.x * (long long)blockDim.x; base < total; base += span) {
-    const long long idx = base + threadIdx.x;
-    uint32_t out[CB];
-    if (idx < total) {
-      const long long wpos = idx % hw_words;
-      const long long t = idx / hw_words;
-      const int chunk = (int)(t % cc);
-      const long long img = t / cc;
-      uint32_t in[CB];
-#pragma unroll
-      for (int k = 0; k < CB; ++k) {
-        const int ch = chunk * CB + k;
-        in[k] = ch < c ? __ldg(src + (img * c + ch) * hw_words + wpos) : 0u;
-      }
-      transpose_words<EB, CB>(in, out);
-    }
-    if constexpr (NP == 1) {
-      if (idx < total) reinterpret_cast<uint4 *>(dst)[idx] = make_uint4(out[0], out[1], out[2], out[3]);
-    } else {
-      if (idx < total) {
-#pragma unroll
-        for (int q = 0; q < NP; ++q)
-          stage[q * (kPackThreads + kPackPad) + threadIdx.x] = make_uint4(out[4 * q], out[4 * q + 1], out[4 * q + 2], out[4 * q + 3]);
-      }
-      __syncthreads();
-      // piece k of the block's output (k = thread * NP + piece) is stored by thread k % 256 in round k / 256
-      uint4 *d4 = reinterpret_cast<uint4 *>(dst) + base * NP;
-      const long long pieces = (total - base < blockDim.x ? total - base : blockDim.x) * NP;
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const int k = i * kPackThreads + threadIdx.x;
-        if (k < pieces) d4[k] = stage[(k % NP) * (kPackThreads + kPackPad) + k / NP];
-      }
-      __syncthreads();
-    }
-  }
-}
-
-template <int EB, int CB>
-__global__ void nchwc_to_nchw_vec_kernel(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, int n, int c,
-                                         int cb_total, long long hw_words) {
-  // cb_total = stored channel blocks of the source; only the first c channels are written
-  const long long total = (long long)n * cb_total * hw_words;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long wpos = idx % hw_words;
-    const long long t = idx / hw_words;
-    const int chunk = (int)(t % cb_total);
-    const long long img = t / cb_total;
-    if (chunk * CB >= c) continue;
-    uint32_t in[CB], out[CB];
-    const uint4 *s4 = reinterpret_cast<const uint4 *>(src + idx * CB);
-#pragma unroll
-    for (int q = 0; q < CB / 4; ++q) {
-      const uint4 v = __ldg(s4 + q);
-      in[4 * q] = v.x; in[4 * q + 1] = v.y; in[4 * q + 2] = v.z; in[4 * q + 3] = v.w;
-    }
-    untranspose_words<EB, CB>(in, out);
-#pragma unroll
-    for (int k = 0; k < CB; ++k) {
-      const int ch = chunk * CB + k;
-      if (ch < c) dst[(img * c + ch) * hw_words + wpos] = out[k];
-    }
-  }
-}
-
-// element loops: any shape
-template <typename T>
-__global__ void nchw_to_nchwc_kernel(const T *__restrict__ src, T *__restrict__ dst, int n, int c, int h, int w,
-                                     int cb) {
-  // one thread = one (pixel, channel block): reads cb strided values, writes cb contiguous
-  const int cc = (c + cb - 1) / cb;
-  const long long hw = (long long)h * w;
-  const long long total = (long long)n * cc * hw;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long pix = idx % hw;
-    const long long t = idx / hw;
-    const int chunk = (int)(t % cc);
-    const long long img = t / cc;
-    T *d = dst + idx * cb;
-    for (int k = 0; k < cb; ++k) {
-      const int ch = chunk * cb + k;
-      d[k] = ch < c ? src[(img * c + ch) * hw + pix] : T(0);
-    }
-  }
-}
-
-template <typename T>
-__global__ void nchwc_to_nchw_kernel(const T *__restrict__ src, T *__restrict__ dst, int n, int c, int h, int w,
-                                     int cb) {
-  const int cc = (c + cb - 1) / cb;
-  const long long hw = (long long)h * w;
-  const long long total = (long long)n * c * hw;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long pix = idx % hw;
-    const long long t = idx / hw;
-    const int ch = (int)(t % c);
-    const long long img = t / c;
-    dst[idx] = src[((img * cc + ch / cb) * hw + pix) * cb + ch % cb];
-  }
-}
-
 __global__ void oihw_to_ref_i8_kernel(const int8_t *__restrict__ src, int8_t *__restrict__ dst, int o, int i, int kh,
                                       int kw, int cb) {
   const int oc = (o + 15) / 16, icc = (i + cb - 1) / cb, c4 = cb / 4;
@@ -1482,15 +1309,74 @@ static int static_scratch_address(void **out) {
 }
 
 template <int EB, int CB>
-static void launch_pack_vec(const void *src, void *dst, int n, int c, long long hw_words, cudaStream_t st) {
-  const long long total = (long long)n * ((c + CB - 1) / CB) * hw_words;
-  nchw_to_nchwc_vec_kernel<EB, CB><<<grid_for(total), kPackThreads, 0, st>>>(static_cast<const uint32_t *>(src), static_cast<uint32_t *>(dst), n, c, hw_words);
+static int launch_layout(bool pack, const void *src, void *dst, int n, int c, long long hw, cudaStream_t st) {
+  LayoutParams p{};
+  p.src = static_cast<const uint8_t *>(src);
+  p.dst = static_cast<uint8_t *>(dst);
+  p.c = c; p.cc = (c + CB - 1) / CB; p.hw = hw;
+  const long long image = (long long)c * hw * EB, blocked_image = (long long)p.cc * hw * CB * EB;
+  if ((long long)n * p.cc > (1ll << 30) && n > 1) {  // unit numbers are 31 bits: very many units go in two halves
+    const int half = n / 2;
+    const int rc = launch_layout<EB, CB>(pack, src, dst, half, c, hw, st);
+    if (rc) return rc;
+    return launch_layout<EB, CB>(pack, p.src + half * (pack ? image : blocked_image), p.dst + half * (pack ? blocked_image : image), n - half,
+                                 c, hw, st);
+  }
+  p.units = n * p.cc;
+  const long long nchw = n * image, blocked = n * blocked_image;
+  p.src_bytes = pack ? nchw : blocked;
+  p.dst_bytes = pack ? blocked : nchw;
+  p.div_cc = make_fast_div((uint32_t)p.cc);
+  if ((CB == 16 || EB == 1) && !pack && hw * EB % 4 == 0 && aligned16(src) && aligned16(dst)) {
+    const long long words = hw * EB / 4;
+    nchwc_to_nchw_words_kernel<EB, CB><<<grid_for(p.units * words), kLayoutThreads, 0, st>>>(p, words);
+    g_launches.fetch_add(1);
+    return cudaGetLastError() == cudaSuccess ? UNIT_OK : UNIT_ERR_LAUNCH;
+  }
+  // tiles of 16 KB, smaller (down to 4 KB) where that is needed to give every SM a few of them
+  long long tile = kLayoutTileBytes;
+  while (tile > 4096 && blocked / tile < 4 * 148) tile /= 2;
+  const long long unit_bytes = (long long)CB * hw * EB;
+  long long blocks, staged;
+  // Blocked -> NCHW keeps whole units up to 44 KB (the shared memory of a block without an opt-in): their result is one
+  // run, where every row of a span begins and ends inside a vector that it shares with another block.
+  if (unit_bytes <= (pack ? tile + tile / 4 : 45056)) {
+    p.group = (int)(tile / unit_bytes > 1 ? tile / unit_bytes : 1);
+    blocks = (p.units + p.group - 1) / p.group;
+    staged = p.group * unit_bytes + 32;
+  } else {
+    const int most = (int)(tile / (CB * EB));
+    const long long spans = (hw + most - 1) / most;
+    p.span = round_up((int)((hw + spans - 1) / spans), 16);
+    p.spans = (int)((hw + p.span - 1) / p.span);
+    blocks = (long long)p.units * p.spans;
+    staged = CB * ((long long)p.span * EB + 16);
+  }
+  if (blocks > 0x7fffffffll) return UNIT_ERR_TOO_LARGE;
+  p.div_hw = make_fast_div((uint32_t)(p.group > 0 ? hw : 1));
+  p.div_spans = make_fast_div((uint32_t)(p.spans > 0 ? p.spans : 1));
+  if (pack) {
+    nchw_to_nchwc_kernel<EB, CB><<<(unsigned)blocks, kLayoutThreads, (size_t)staged, st>>>(p);
+  } else {
+    nchwc_to_nchw_kernel<EB, CB><<<(unsigned)blocks, kLayoutThreads, (size_t)staged, st>>>(p);
+  }
+  g_launches.fetch_add(1);
+  return cudaGetLastError() == cudaSuccess ? UNIT_OK : UNIT_ERR_LAUNCH;
 }
-template <int EB, int CB>
-static void launch_unpack_vec(const void *src, void *dst, int n, int c, long long hw_words, cudaStream_t st) {
-  const int cb_total = (c + CB - 1) / CB;
-  const long long total = (long long)n * cb_total * hw_words;
-  nchwc_to_nchw_vec_kernel<EB, CB><<<grid_for(total), 256, 0, st>>>(static_cast<const uint32_t *>(src), static_cast<uint32_t *>(dst), n, c, cb_total, hw_words);
+static int run_layout(bool pack, const void *src, void *dst, int n, int c, int h, int w, int cb, int eb, cudaStream_t st) {
+  if (!src || !dst) return UNIT_ERR_NULL;
+  if (n < 1 || c < 1 || h < 1 || w < 1) return UNIT_ERR_SHAPE;
+  if (cb != 4 && cb != 16) return UNIT_ERR_LAYOUT;
+  if (eb != 1 && eb != 2 && eb != 4) return UNIT_ERR_LAYOUT;
+  const long long hw = (long long)h * w;
+  if (cb == 16) {
+    if (eb == 1) return launch_layout<1, 16>(pack, src, dst, n, c, hw, st);
+    if (eb == 2) return launch_layout<2, 16>(pack, src, dst, n, c, hw, st);
+    return launch_layout<4, 16>(pack, src, dst, n, c, hw, st);
+  }
+  if (eb == 1) return launch_layout<1, 4>(pack, src, dst, n, c, hw, st);
+  if (eb == 2) return launch_layout<2, 4>(pack, src, dst, n, c, hw, st);
+  return launch_layout<4, 4>(pack, src, dst, n, c, hw, st);
 }
 
 }  // namespace unit
@@ -1995,62 +1881,12 @@ int unit_gemm_f16f32(int32_t m, int32_t n, int32_t k, const void *a, int64_t lda
 // ---- layout transforms ---------------------------------------------------------
 int unit_pack_data_nchw_to_nchwc(const void *src, void *dst, int32_t n, int32_t c, int32_t h, int32_t w, int32_t cb,
                                  int32_t eb, void *stream) {
-  if (!src || !dst) return UNIT_ERR_NULL;
-  if (n < 1 || c < 1 || h < 1 || w < 1) return UNIT_ERR_SHAPE;
-  if (cb != 4 && cb != 16) return UNIT_ERR_LAYOUT;
-  if (eb != 1 && eb != 2 && eb != 4) return UNIT_ERR_LAYOUT;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long hw = (long long)h * w;
-  if (hw * eb % 4 == 0 && aligned16(src) && aligned16(dst)) {
-    // register transpose of 4-byte words, 16-byte stores
-    const long long hww = hw * eb / 4;
-    if (cb == 16) {
-      if (eb == 1) launch_pack_vec<1, 16>(src, dst, n, c, hww, st);
-      else if (eb == 2) launch_pack_vec<2, 16>(src, dst, n, c, hww, st);
-      else launch_pack_vec<4, 16>(src, dst, n, c, hww, st);
-    } else {
-      if (eb == 1) launch_pack_vec<1, 4>(src, dst, n, c, hww, st);
-      else if (eb == 2) launch_pack_vec<2, 4>(src, dst, n, c, hww, st);
-      else launch_pack_vec<4, 4>(src, dst, n, c, hww, st);
-    }
-  } else {
-    const long long total = (long long)n * ((c + cb - 1) / cb) * hw;
-    const unsigned g = grid_for(total);
-    if (eb == 1) nchw_to_nchwc_kernel<uint8_t><<<g, 256, 0, st>>>((const uint8_t *)src, (uint8_t *)dst, n, c, h, w, cb);
-    else if (eb == 2) nchw_to_nchwc_kernel<uint16_t><<<g, 256, 0, st>>>((const uint16_t *)src, (uint16_t *)dst, n, c, h, w, cb);
-    else nchw_to_nchwc_kernel<uint32_t><<<g, 256, 0, st>>>((const uint32_t *)src, (uint32_t *)dst, n, c, h, w, cb);
-  }
-  g_launches.fetch_add(1);
-  return cudaGetLastError() == cudaSuccess ? UNIT_OK : UNIT_ERR_LAUNCH;
+  return run_layout(true, src, dst, n, c, h, w, cb, eb, static_cast<cudaStream_t>(stream));
 }
 
 int unit_unpack_data_nchwc_to_nchw(const void *src, void *dst, int32_t n, int32_t c, int32_t h, int32_t w, int32_t cb,
                                    int32_t eb, void *stream) {
-  if (!src || !dst) return UNIT_ERR_NULL;
-  if (n < 1 || c < 1 || h < 1 || w < 1) return UNIT_ERR_SHAPE;
-  if (cb != 4 && cb != 16) return UNIT_ERR_LAYOUT;
-  if (eb != 1 && eb != 2 && eb != 4) return UNIT_ERR_LAYOUT;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long hw = (long long)h * w;
-  if (hw * eb % 4 == 0 && aligned16(src) && aligned16(dst)) {
-    const long long hww = hw * eb / 4;
-    if (cb == 16) {
-      if (eb == 1) launch_unpack_vec<1, 16>(src, dst, n, c, hww, st);
-      else if (eb == 2) launch_unpack_vec<2, 16>(src, dst, n, c, hww, st);
-      else launch_unpack_vec<4, 16>(src, dst, n, c, hww, st);
-    } else {
-      if (eb == 1) launch_unpack_vec<1, 4>(src, dst, n, c, hww, st);
-      else if (eb == 2) launch_unpack_vec<2, 4>(src, dst, n, c, hww, st);
-      else launch_unpack_vec<4, 4>(src, dst, n, c, hww, st);
-    }
-  } else {
-    const unsigned g = grid_for((long long)n * c * hw);
-    if (eb == 1) nchwc_to_nchw_kernel<uint8_t><<<g, 256, 0, st>>>((const uint8_t *)src, (uint8_t *)dst, n, c, h, w, cb);
-    else if (eb == 2) nchwc_to_nchw_kernel<uint16_t><<<g, 256, 0, st>>>((const uint16_t *)src, (uint16_t *)dst, n, c, h, w, cb);
-    else nchwc_to_nchw_kernel<uint32_t><<<g, 256, 0, st>>>((const uint32_t *)src, (uint32_t *)dst, n, c, h, w, cb);
-  }
-  g_launches.fetch_add(1);
-  return cudaGetLastError() == cudaSuccess ? UNIT_OK : UNIT_ERR_LAUNCH;
+  return run_layout(false, src, dst, n, c, h, w, cb, eb, static_cast<cudaStream_t>(stream));
 }
 
 int unit_pack_weights_oihw_to_ref_i8(const int8_t *src, int8_t *dst, int32_t o, int32_t i, int32_t kh, int32_t kw,
