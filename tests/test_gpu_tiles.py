@@ -33,11 +33,11 @@ def launched(run):
 def dense_case(U, m, n, k, seed=0):
     rng = np.random.default_rng(m + n + k + seed)
     a = rng.integers(0, 256, (m, k), dtype=np.uint8)
-    b = rng.integers(-128, 128, (k, n), dtype=np.int8)
+    b = rng.integers(-128, 128, (n, k), dtype=np.int8)
     got, names = launched(lambda: U.dense_dotprod(dev(a), dev(no.pack_dense_weights(b, 16))))
     U.device_status()
     # (float64 holds these integer sums exactly: |sum| <= 255 * 128 * k < 2^53)
-    want = (dev(a).double() @ dev(b).double()).to(torch.int32)
+    want = (dev(a).double() @ dev(b).double().t()).to(torch.int32)
     assert torch.equal(got, want)
     return names
 
@@ -65,3 +65,29 @@ def test_dense_reductions_that_end_inside_a_stage(U, m, n, k):
 @pytest.mark.parametrize('n,k', [(272, 1024), (272, 1032), (48, 1016), (2064, 520), (16, 56), (528, 72), (528, 456)])
 def test_gemm_reductions_that_end_inside_a_stage(U, m, n, k):
     gemm_case(U, m, n, k)
+
+
+# (batch, chunks, depth, h, w, c_out, kernel, padding): one and two sub-tiles, padding in no and in every dimension,
+# kernels that are flat in one dimension, slices smaller than a tile, a column block that is not full
+@pytest.mark.parametrize('n,c,d,h,w,co,k,p', [
+    (4, 64, 18, 44, 44, 64, (3, 3, 3), (0, 0, 0)),
+    (3, 32, 9, 30, 30, 48, (3, 3, 3), (1, 1, 1)),
+    (2, 32, 40, 34, 30, 32, (2, 3, 1), (1, 0, 0)),
+    (5, 64, 6, 58, 58, 16, (1, 3, 3), (0, 1, 1)),
+    (2, 32, 17, 23, 61, 80, (3, 1, 3), (2, 0, 1)),
+])
+def test_conv3d_windows_over_the_whole_batch(U, n, c, d, h, w, co, k, p):
+    from oracle import c_oracle
+    rng = np.random.default_rng(n + c + d + h + co)
+    x = rng.integers(0, 256, (n, c // 16, d, h, w, 16), dtype=np.uint8)
+    wt = rng.integers(-128, 128, (co // 16, c // 16) + k + (4, 16, 4), dtype=np.int8)
+    b = rng.integers(-2 ** 15, 2 ** 15, co, dtype=np.int32)
+    ref = c_oracle.conv3d_u8s8(x, wt, (1, 1, 1), p, bias=b)
+    xd, wd, bd = dev(x), dev(wt), dev(b)
+    got, names = launched(lambda: U.conv3d_NCDHWc_int8(xd, wd, stride=1, padding=p, bias=bd))
+    U.device_status()
+    assert any('A_CONV_WIN' in v for v in names), names
+    assert np.array_equal(got.cpu().numpy(), ref)
+    gotq = U.conv3d_NCDHWc_int8(xd, wd, stride=1, padding=p, bias=bd, requant_shift=10)
+    assert np.array_equal(gotq.cpu().numpy(), np.clip((ref.astype(np.int64) + 512) >> 10, 0, 255).astype(np.uint8))
+    U.device_status()

@@ -172,6 +172,12 @@ struct IgemmParams {
   int win_wp, win_rows, win_bytes, win_tpi;  // win_bytes: distance between the two windows of a stage (a multiple of 128)
   int win_box_bytes;                         // bytes one window copy delivers: win_rows * win_wp * 16
   FastDiv div_wp, div_tpi;
+  // Window form in three dimensions (win_od > 0): the tiles run over the output slices (image, od) of the whole batch
+  // (win_tpi tiles per slice, n_img slices), the K loop over (kd, chunk pair), and the windows of kernel depth kd
+  // come from input depth od + kd - pd through a five-dimensional map.  win_pairs: chunk pairs per kd.
+  int win_od, win_pairs;
+  FastDiv div_od, div_pairs;
+  long long out_batch_stride;  // between images of the batch, in units of 16 output elements
   // Convolution in three dimensions (one image, [c/16][D][H][W][16]): the depth axis takes the place of
   // the image axis of the two-dimensional kernel (a 128-row tile then runs over (od, oh, ow)), kernel
   // depth KD adds a third tap index, and the output strides below place (od, channel group).
@@ -1039,6 +1045,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         const uint32_t img = fast_div((uint32_t)m_tile, p.div_tpi);
         const uint32_t q0 = ((uint32_t)m_tile - img * (uint32_t)p.win_tpi) * (uint32_t)(kTileM * MT);
         const int y0 = (int)fast_div(q0, p.div_wp) - p.ph;
+        const uint32_t bat = p.win_od > 0 ? fast_div(img, p.div_od) : 0u;
+        const int z0 = p.win_od > 0 ? (int)(img - bat * (uint32_t)p.win_od) - p.pd : 0;
         for (int ks = ks_begin; ks < ks_end; ++ks) {
           if (!mbar_wait_warp(smem_u32(&ps->empty[s]), ring_phase ^ 1u, wc, kErrWaitEmpty)) {
             alive = false;
@@ -1047,7 +1055,11 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           const uint32_t bar = smem_u32(&ps->full[s]);
           if (tx_poster) mbar_arrive_expect_tx(bar, 2u * (uint32_t)p.win_box_bytes);
           __syncwarp();
-          if (lane == 0 && copy_id < 2)
+          if (lane == 0 && copy_id < 2 && p.win_od > 0) {
+            const int kd = (int)fast_div((uint32_t)ks, p.div_pairs);
+            tma_tile_5d(smem_base + s * stage_bytes + (uint32_t)copy_id * (uint32_t)p.win_bytes, &tmap, -2 * p.pw, y0, z0 + kd,
+                        2 * (ks - kd * p.win_pairs) + copy_id, (int)bat, bar);
+          } else if (lane == 0 && copy_id < 2)
             tma_tile_4d(smem_base + s * stage_bytes + (uint32_t)copy_id * (uint32_t)p.win_bytes, &tmap, -2 * p.pw, y0,
                         2 * ks + copy_id, (int)img, bar);
           if (++s == (uint32_t)p.stages) { s = 0; ring_phase ^= 1u; }
@@ -1397,7 +1409,12 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         const uint32_t oh = fast_div(q, p.div_wp);
         const uint32_t ow = q - oh * (uint32_t)p.win_wp;
         mvalid = (int)ow < p.OW && (int)oh < p.OH && (int)img < p.n_img;
-        obase = ((long long)img * p.out_img_stride + (long long)n_tile * (p.bn >> 4) * p.out_grp_stride + (long long)oh * p.OW + ow) * 16;
+        long long place = (long long)img * p.out_img_stride;
+        if (p.win_od > 0) {
+          const uint32_t bat = fast_div(img, p.div_od);
+          place = (long long)bat * p.out_batch_stride + (long long)(img - bat * (uint32_t)p.win_od) * p.out_img_stride;
+        }
+        obase = (place + (long long)n_tile * (p.bn >> 4) * p.out_grp_stride + (long long)oh * p.OW + ow) * 16;
       } else if constexpr (EPI == EPI_RAW_ROWS) {
         obase = m * p.ldc + (long long)n_tile * p.bn;
       } else {

@@ -323,6 +323,7 @@ struct PackParams {
   uint4 *dst;
   int mode, n_total, bn, kc, cols, k_stages, n_tiles;
   int Cc, KH, KW, kwg;  // conv
+  int win_pairs, win_kh;  // PACK_CONV_WIN: chunk pairs (stages) per kernel depth, rows of the kernel
   int tw, sft_h, sft_w;  // PACK_STEM_S2D: taps per row of the 2x2-folded kernel, tap shifts
   int pair_g, pair_qmin, pair_pad;  // PACK_CONV_PAIR: pair offsets per kernel row, the first offset, the horizontal padding
   int K, T;             // dense / gemm (K in elements)
@@ -350,8 +351,10 @@ __global__ void pack_weights_kernel(const PackParams p) {
         for (int m = 0; m < 4; ++m) w[m] = *reinterpret_cast<const uint32_t *>(s + m * 64);
       } else if (p.mode == PACK_CONV_WIN) {
         // window form: stage = pair of channel chunks; within it, columns (tap, chunk 2 ks) and (tap, chunk 2 ks + 1)
-        const int tap = jj >> 1, ci = 2 * ks + (jj & 1);
-        const int kh = tap / p.KW, kw = tap % p.KW;
+        // (three dimensions: stages run (kd, pair), and KH counts the kernel's kd * kh rows)
+        const int kd = ks / p.win_pairs;
+        const int tap = jj >> 1, ci = 2 * (ks - kd * p.win_pairs) + (jj & 1);
+        const int kh = kd * p.win_kh + tap / p.KW, kw = tap % p.KW;
         const uint8_t *s = p.src + ((((size_t)(oc >> 4) * p.Cc + ci) * p.KH + kh) * p.KW + kw) * 256 + (oc & 15) * 4;
         for (int m = 0; m < 4; ++m) w[m] = *reinterpret_cast<const uint32_t *>(s + m * 64);
       } else if (p.mode == PACK_CONV_PAIR) {
@@ -966,6 +969,25 @@ static bool make_box_map(CUtensorMap *map, int n, int c_in, int h, int w, const 
   return r == CUDA_SUCCESS;
 }
 
+// The window form's map in three dimensions: u8 [n][c/16][d][h][w][16] seen as (8-byte units of a pixel row, image
+// row, depth, channel chunk, image); one copy fetches `rows` rows of `wp` pixels, zero-filled outside the image.
+static bool make_win_map_3d(CUtensorMap *map, const unit_conv3d_desc *d, const void *x, const WinGeom &g) {
+  typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                               const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static EncodeFn encode = driver_fn<EncodeFn>("cuTensorMapEncodeTiled");
+  const cuuint64_t H = (cuuint64_t)d->h, W = (cuuint64_t)d->w, D = (cuuint64_t)d->d, C = (cuuint64_t)(d->c_in / 16);
+  if (!encode || !tensor_map_allowed((long long)d->n * d->c_in * d->d * d->h * d->w)) return false;
+  const cuuint64_t dims[5] = {W * 2, H, D, C, (cuuint64_t)d->n};
+  const cuuint64_t strides[4] = {W * 16, H * W * 16, D * H * W * 16, C * D * H * W * 16};
+  const cuuint32_t box[5] = {(cuuint32_t)g.wp * 2, (cuuint32_t)g.rows, 1, 1, 1};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 5, const_cast<void *>(x), dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 // Tiled-mode tensor map over a row-major matrix of `row_bytes` used bytes per row and `ld` bytes
 // between rows, seen as (8-byte half of a K column, K column, row): one copy fetches one 16-byte K
 // column of 128 consecutive rows, which lands in shared memory as that column's core matrices.
@@ -1251,15 +1273,8 @@ static TileCfg conv3d_cfg(const unit_conv3d_desc *d) {
   return make_cfg(d->c_out, d->kd * d->kh * d->kw * (d->c_in / 16), cheap);
 }
 
-// Plan for image `img` of the batch.  The depth axis takes the place of the two-dimensional kernel's
-// image axis: a 128-row tile runs over (od, oh, ow) of one image.
-static int plan_conv3d_i8(PlanImpl &pl, const unit_conv3d_desc *d, const uint8_t *x, const void *pw, const EpilogueArgs &e,
-                          void *out) {
-  const TileCfg c = conv3d_cfg(d);
-  const int epi = e.out_u8 ? (e.residual ? EPI_RES_NCHWC : EPI_REQ_NCHWC) : (e.mul != 1 ? EPI_MUL_NCHWC : EPI_RAW_NCHWC);
-  pl = PlanImpl{};
-  IgemmParams &p = pl.p;
-  p.a = x; p.b = static_cast<const uint8_t *>(pw); p.out = out; p.bias = e.bias; p.shift = e.shift;
+static void fill_conv3d(IgemmParams &p, const unit_conv3d_desc *d, const void *x, const EpilogueArgs &e, void *out) {
+  p.a = static_cast<const uint8_t *>(x); p.out = out; p.bias = e.bias; p.shift = e.shift;
   p.mul = e.mul; p.residual = e.residual; p.a_signed = e.x_signed ? 1 : 0;
   p.H = d->h; p.W = d->w; p.Cc = d->c_in / 16;
   p.KD = d->kd; p.KH = d->kh; p.KW = d->kw;
@@ -1281,6 +1296,88 @@ static int plan_conv3d_i8(PlanImpl &pl, const unit_conv3d_desc *d, const uint8_t
   p.src_imgs = d->d;
   p.n_img = OD;
   p.acc_bound = 255ll * 128ll * d->c_in * d->kd * d->kh * d->kw;
+}
+
+// The two-dimensional convolution over one depth slice of the kernel, with the batch's N * OD output slices as images.
+static unit_conv_desc conv3d_slices(const unit_conv3d_desc *d) {
+  unit_conv_desc s{};
+  s.n = d->n * ((d->d + 2 * d->pad_d - d->kd) / d->stride_d + 1);
+  s.c_in = d->c_in; s.h = d->h; s.w = d->w; s.c_block = 16; s.c_out = d->c_out;
+  s.kh = d->kh; s.kw = d->kw; s.stride_h = d->stride_h; s.stride_w = d->stride_w; s.pad_h = d->pad_h; s.pad_w = d->pad_w;
+  return s;
+}
+// Window form in three dimensions: weight-side eligibility and the tile shape of the packed copy (one stage per
+// kernel depth and pair of channel chunks).
+static bool win3d_weights_ok(const unit_conv3d_desc *d) {
+  const unit_conv_desc s = conv3d_slices(d);
+  return d->stride_d == 1 && win_weights_ok(&s);
+}
+static TileCfg win3d_cfg(const unit_conv3d_desc *d) {
+  TileCfg c = conv3d_cfg(d);
+  const int taps = d->kh * d->kw;
+  c.kc = 2 * taps;
+  c.cols_pad = c.cols;
+  c.k_stages = d->kd * (d->c_in / 32);
+  c.last_ksteps = taps;
+  c.b_stage_bytes = (size_t)c.kc * c.bn * 16;
+  return c;
+}
+
+// Window-form plan for the whole batch; returns false where the form does not apply (the caller then plans one
+// launch per image).  The box and im2col forms copy a 16-byte pixel row per tap: 27 x 4 copies of 2 KB for a
+// 128-row sub-tile of a 3x3x3 kernel on 64 channels, and the copy engine's work per row bounds them; the window
+// form makes 3 x 4 copies of the rows a tile touches (3x3x3 64->64, 4 x 16 x 58 x 58: 85.4 -> 34.2 us in one launch).
+static bool plan_conv3d_win(PlanImpl &pl, const unit_conv3d_desc *d, const void *x, const void *pw, const EpilogueArgs &e, void *out,
+                            int *rc) {
+  if (!use_tma() || !win3d_weights_ok(d)) return false;
+  const long long od = d->d + 2 * d->pad_d - d->kd + 1, slices = d->n * od;
+  if (slices >= (1ll << 24)) return false;
+  const unit_conv_desc s2 = conv3d_slices(d);
+  const TileCfg wc = win3d_cfg(d);
+  const int sms = sm_count();
+  for (int mt = 2; mt >= 1; --mt) {
+    const WinGeom g = win_geom(&s2, mt, wc);
+    const long long tiles = slices * g.tpi * wc.n_tiles;
+    if (!g.ok || tiles < (mt == 2 ? 2 : 1) * (long long)sms || tiles * kTileM * mt >= (1ll << 31)) continue;
+    CUtensorMap map;
+    if (!make_win_map_3d(&map, d, x, g)) return false;
+    const TileCfg c = conv3d_cfg(d);
+    pl = PlanImpl{};
+    fill_conv3d(pl.p, d, x, e, out);
+    IgemmParams &p = pl.p;
+    p.b = static_cast<const uint8_t *>(pw) + (size_t)c.n_tiles * c.k_stages * c.b_stage_bytes;  // the second packed copy
+    p.win_wp = g.wp; p.win_rows = g.rows; p.win_bytes = g.bytes; p.win_box_bytes = g.box_bytes; p.win_tpi = g.tpi;
+    p.div_wp = make_fast_div((uint32_t)g.wp);
+    p.div_tpi = make_fast_div((uint32_t)g.tpi);
+    p.win_od = (int)od;
+    p.win_pairs = d->c_in / 32;
+    p.div_od = make_fast_div((uint32_t)od);
+    p.div_pairs = make_fast_div((uint32_t)p.win_pairs);
+    p.out_batch_stride = (long long)(d->c_out / 16) * p.out_grp_stride;
+    p.n_img = (int)slices;
+    p.m_total = slices * g.tpi * kTileM * mt;
+    pl.table_mt = mt;
+    pl.table_ksplit = 1;
+    TileCfg wcm = wc;
+    wcm.a_stage_bytes = 2 * (size_t)g.bytes;
+    const int epi = e.out_u8 ? (e.residual ? EPI_RES_NCHWC : EPI_REQ_NCHWC) : (e.mul != 1 ? EPI_MUL_NCHWC : EPI_RAW_NCHWC);
+    *rc = prepare_conv_i8<A_CONV_WIN>(pl, wcm, epi, &map);
+    return true;
+  }
+  return false;
+}
+
+// Plan for image `img` of the batch.  The depth axis takes the place of the two-dimensional kernel's
+// image axis: a 128-row tile runs over (od, oh, ow) of one image.
+static int plan_conv3d_i8(PlanImpl &pl, const unit_conv3d_desc *d, const uint8_t *x, const void *pw, const EpilogueArgs &e,
+                          void *out) {
+  const TileCfg c = conv3d_cfg(d);
+  const int epi = e.out_u8 ? (e.residual ? EPI_RES_NCHWC : EPI_REQ_NCHWC) : (e.mul != 1 ? EPI_MUL_NCHWC : EPI_RAW_NCHWC);
+  pl = PlanImpl{};
+  fill_conv3d(pl.p, d, x, e, out);
+  IgemmParams &p = pl.p;
+  p.b = static_cast<const uint8_t *>(pw);
+  const int OD = p.n_img;
   CUtensorMap map;
   if (use_tma() && d->stride_d == 1 && d->stride_h == 1 && d->stride_w == 1) {
     const BoxGeom g = choose_box(OD, p.OH, p.OW);
@@ -1522,6 +1619,7 @@ int unit_pack_weights_conv_i8(const unit_conv_desc *d, const int8_t *w, void *pa
     PackParams pwn = pp;
     pwn.dst = reinterpret_cast<uint4 *>(static_cast<uint8_t *>(packed) + (size_t)c.n_tiles * c.k_stages * c.b_stage_bytes);
     pwn.mode = PACK_CONV_WIN;
+    pwn.win_pairs = wc.k_stages; pwn.win_kh = d->kh;
     pwn.bn = wc.bn; pwn.kc = wc.kc; pwn.cols = wc.cols; pwn.k_stages = wc.k_stages; pwn.n_tiles = wc.n_tiles;
     rc = launch_pack(pwn, static_cast<cudaStream_t>(stream));
   }
@@ -1712,7 +1810,12 @@ int unit_conv2d_run(const unit_conv_plan *plan, void *stream) {
 size_t unit_packed_weights_bytes_conv3d_i8(const unit_conv3d_desc *d) {
   if (check_conv3d(d)) return 0;
   const TileCfg c = conv3d_cfg(d);
-  return (size_t)c.n_tiles * c.k_stages * c.b_stage_bytes;
+  size_t bytes = (size_t)c.n_tiles * c.k_stages * c.b_stage_bytes;
+  if (win3d_weights_ok(d)) {  // second copy in the window form's column order
+    const TileCfg wc = win3d_cfg(d);
+    bytes += (size_t)wc.n_tiles * wc.k_stages * wc.b_stage_bytes;
+  }
+  return bytes;
 }
 
 int unit_pack_weights_conv3d_i8(const unit_conv3d_desc *d, const int8_t *w, void *packed, void *stream) {
@@ -1728,7 +1831,16 @@ int unit_pack_weights_conv3d_i8(const unit_conv3d_desc *d, const int8_t *w, void
   pp.n_total = d->c_out; pp.bn = c.bn; pp.kc = c.kc; pp.cols = c.cols; pp.k_stages = c.k_stages; pp.n_tiles = c.n_tiles;
   // [c_out/16][c_in/16][kd][kh][kw][4][16][4]: the depth and height taps form one axis of kd * kh entries
   pp.Cc = d->c_in / 16; pp.KH = d->kd * d->kh; pp.KW = d->kw;
-  return launch_pack(pp, static_cast<cudaStream_t>(stream));
+  rc = launch_pack(pp, static_cast<cudaStream_t>(stream));
+  if (rc == UNIT_OK && win3d_weights_ok(d)) {
+    const TileCfg wc = win3d_cfg(d);
+    pp.dst = reinterpret_cast<uint4 *>(static_cast<uint8_t *>(packed) + (size_t)c.n_tiles * c.k_stages * c.b_stage_bytes);
+    pp.mode = PACK_CONV_WIN;
+    pp.kc = wc.kc; pp.k_stages = wc.k_stages;
+    pp.win_pairs = d->c_in / 32; pp.win_kh = d->kh;
+    rc = launch_pack(pp, static_cast<cudaStream_t>(stream));
+  }
+  return rc;
 }
 
 int unit_conv3d_int8_ncdhwc(const unit_conv3d_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out,
@@ -1747,6 +1859,10 @@ int unit_conv3d_int8_ncdhwc(const unit_conv3d_desc *d, const void *x, const void
   const long long od = (d->d + 2 * d->pad_d - d->kd) / d->stride_d + 1, oh = (d->h + 2 * d->pad_h - d->kh) / d->stride_h + 1,
                   ow = (d->w + 2 * d->pad_w - d->kw) / d->stride_w + 1;
   const long long out_elems = od * oh * ow * d->c_out;
+  {
+    PlanImpl pl;
+    if (plan_conv3d_win(pl, d, x, pw, e, out, &rc)) return rc ? rc : run_plan(pl, static_cast<cudaStream_t>(stream));
+  }
   for (int img = 0; img < d->n; ++img) {  // one launch per image
     EpilogueArgs ei = e;
     if (e.residual) ei.residual = e.residual + img * out_elems;
