@@ -91,3 +91,22 @@ def test_conv3d_windows_over_the_whole_batch(U, n, c, d, h, w, co, k, p):
     gotq = U.conv3d_NCDHWc_int8(xd, wd, stride=1, padding=p, bias=bd, requant_shift=10)
     assert np.array_equal(gotq.cpu().numpy(), np.clip((ref.astype(np.int64) + 512) >> 10, 0, 255).astype(np.uint8))
     U.device_status()
+
+
+# every form of the final pack: the shorter one (8), a dot product that scales the residual (up to 15), plain adds
+# above; with one and two sub-tiles per tile, a ragged last column block and sums on both sides of the clamp
+@pytest.mark.parametrize('shift', [1, 7, 8, 9, 15, 16, 23])
+@pytest.mark.parametrize('n,c,h,co', [(9, 32, 23, 48), (32, 64, 28, 272)])
+def test_requantising_drains_at_every_shift(U, n, c, h, co, shift):
+    from oracle import c_oracle
+    rng = np.random.default_rng(n + shift)
+    x = rng.integers(0, 256, (n, c // 16, h, h, 16), dtype=np.uint8)
+    w = rng.integers(-128, 128, (co // 16, c // 16, 1, 1, 4, 16, 4), dtype=np.int8)
+    b = rng.integers(-2 ** 15, 2 ** 15, co, dtype=np.int32)
+    r = rng.integers(0, 256, (n, co // 16, h, h, 16), dtype=np.uint8)
+    for res in (None, r):
+        want = c_oracle.conv2d_i8_ex(x, w, (1, 1), (0, 0), bias=b, requant_shift=shift, residual=res)
+        got = U.conv2d_NCHWc_int8(dev(x), dev(w), bias=dev(b), out_dtype='uint8', requant_shift=shift,
+                                  residual=None if res is None else dev(res))
+        U.device_status()
+        assert np.array_equal(got.cpu().numpy(), want)

@@ -535,6 +535,11 @@ __device__ __forceinline__ uint32_t make_idesc(int bn, int a_signed) {
   return d;
 }
 
+template <bool V>
+struct BoolTag {
+  static constexpr bool value = V;
+};
+
 struct alignas(16) PipeShared {
   int32_t bias[2][2][kBiasSmem];  // [accumulator set][version]: bias (+ rounding constant) where the drain adds it
   int bias_mma[2];                // per accumulator set: the bias goes in through one more MMA K step
@@ -649,20 +654,33 @@ __device__ __forceinline__ uint4 pack16_shift8(const uint32_t *t) {
                        pack_sat_u16((int32_t)t[4 * q + 3], (int32_t)t[4 * q + 2]), 0x7531);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-// The same with a u8 residual added after the shift: clamp((x >> 8) + r, 0, 255) = clamp((x + 256 r) >> 8, 0, 255),
-// so the residual byte joins its sum one byte up and the pack stays as it is.  (x + 256 r cannot leave s32: the
-// host bounds |x| below 2^30 on this path.)
-__device__ __forceinline__ uint4 pack16_shift8_res(const uint32_t *t, uint4 r) {
-  const uint32_t res[4] = {r.x, r.y, r.z, r.w};
+// The same for any other shift (1 .. 23): 16 more shifts per group.
+__device__ __forceinline__ uint4 pack16_shift(const uint32_t *t, int shift) {
   uint32_t w[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint32_t x0 = t[4 * q] + __byte_perm(res[q], 0u, 0x4404), x1 = t[4 * q + 1] + __byte_perm(res[q], 0u, 0x4414);
-    const uint32_t x2 = t[4 * q + 2] + __byte_perm(res[q], 0u, 0x4424), x3 = t[4 * q + 3] + __byte_perm(res[q], 0u, 0x4434);
-    w[q] = __byte_perm(pack_sat_u16((int32_t)x1, (int32_t)x0), pack_sat_u16((int32_t)x3, (int32_t)x2), 0x7531);
-  }
+  for (int q = 0; q < 4; ++q)
+    w[q] = pack_sat_u8((int32_t)t[4 * q + 1] >> shift, (int32_t)t[4 * q] >> shift,
+                       pack_sat_u8((int32_t)t[4 * q + 3] >> shift, (int32_t)t[4 * q + 2] >> shift, 0u));
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
+// A u8 residual added after the shift: (x >> s) + r = (x + (r << s)) >> s, so the residual byte joins its sum s bits
+// up and the packs stay as they are.  (|x| is below 2^30 on this path and r << s below 2^23: no overflow.)  One
+// two-way dot product per value picks the byte, scales it and adds it: lo / hi = 2^s in the half that meets the
+// byte.  Shift 8: 28 instructions per group against 44 with a permute and an add each.
+// (ResNet-50's 1x1 64->256 with residual at batch 32, shift 10: 20.1 -> 16.2 us per launch, most of it because such
+// shifts now take the decision-free loop; at batch 256 the layer is bound by HBM, 97 us either way.)
+__device__ __forceinline__ void add_residual16(uint32_t (&x)[16], const uint32_t *t, uint4 r, int shift) {
+  const uint32_t res[4] = {r.x, r.y, r.z, r.w};
+  const uint32_t even = 1u << shift, odd = even << 16;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    x[4 * q] = __dp2a_lo(even, res[q], t[4 * q]);
+    x[4 * q + 1] = __dp2a_lo(odd, res[q], t[4 * q + 1]);
+    x[4 * q + 2] = __dp2a_hi(even, res[q], t[4 * q + 2]);
+    x[4 * q + 3] = __dp2a_hi(odd, res[q], t[4 * q + 3]);
+  }
+}
+constexpr int kMaxDotShift = 15;  // 2^s is a 16-bit factor
 
 // Epilogue for 16 consecutive columns of one row: v = accumulator words, bias_s = this
 // group's 16 staged bias values in shared memory (bias + rounding constant for the
@@ -1508,8 +1526,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
       // software pipeline: the read of group g + 1 is in flight while group g is processed
       uint32_t va[16], vb[16];
       // The common cases as a loop of their own, with no per-group decisions and one offset that
-      // advances: the accumulator is final (bias inside it, or none) and, when requantising, the
-      // shift is 8.  (Measured on the 1x1 64->256 layer at batch 256: 35 -> 19 instructions per
+      // advances: the accumulator is final (bias inside it, or none).  (Measured on the 1x1 64->256 layer at batch 256: 35 -> 19 instructions per
       // group, 72 -> 52 us; the drain warps' instruction count is what bounds the write-heavy layers.)
       bool drained = false;
       // 32-bit outputs of the kernels that keep no bias in shared memory (fp16, dense): regrouped stores
@@ -1529,7 +1546,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           ok_k[k] = __shfl_sync(0xffffffffu, mvalid ? 1 : 0, src) != 0;
         }
       }
-      if ((EPI == EPI_RAW_ROWS || folded) && (!epi_requantises(EPI) || p.shift == 8)) {
+      if ((EPI == EPI_RAW_ROWS || folded) && (EPI != EPI_RES_NCHWC || p.shift <= kMaxDotShift)) {
         long long o = obase + (long long)g_begin * gstride;
         uint32_t taddr = t_row + (uint32_t)g_begin * 16u;
         int left = g_stop - g_begin;
@@ -1542,47 +1559,46 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           }
           tmem_ld_wait();
         }
-        while (left > 0) {
-          if (left > 1) {
-            tmem_ld16(taddr + 16u, vb);
-            if constexpr (EPI == EPI_RES_NCHWC) {
-              if (mvalid) rb = *reinterpret_cast<const uint4 *>(p.residual + o + gstride);
-            }
-          }
-          if constexpr (EPI == EPI_REQ_NCHWC) {
-            const uint4 w = pack16_shift8(va);
-            if (mvalid) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) + o) = w;
-          } else if constexpr (EPI == EPI_RES_NCHWC) {
-            if (mvalid) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) + o) = pack16_shift8_res(va, ra);
-          } else if constexpr (kRegroup) {
-            store_group16_regrouped(reinterpret_cast<uint32_t *>(p.out), xs, lane, va, o_k, ok_k, o - obase);
-          } else {
-            if (mvalid) finish_group16<EPI>(p, va, o);
-          }
-          tmem_ld_wait();
-          if (left > 2) {
-            tmem_ld16(taddr + 32u, va);
-            if constexpr (EPI == EPI_RES_NCHWC) {
-              if (mvalid) ra = *reinterpret_cast<const uint4 *>(p.residual + o + 2 * gstride);
-            }
-          }
-          if (left > 1) {
-            if constexpr (EPI == EPI_REQ_NCHWC) {
-              const uint4 w = pack16_shift8(vb);
-              if (mvalid) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) + o + gstride) = w;
-            } else if constexpr (EPI == EPI_RES_NCHWC) {
-              if (mvalid) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) + o + gstride) = pack16_shift8_res(vb, rb);
+        // (the loop exists twice where the shift matters, so that shift 8 keeps its shorter pack)
+        auto drain_final = [&](auto shift8) {
+          constexpr bool kShift8 = decltype(shift8)::value;
+          auto group = [&](const uint32_t *v, const uint4 &res, long long og) {
+            if constexpr (epi_requantises(EPI)) {
+              uint32_t x[16];
+              if constexpr (EPI == EPI_RES_NCHWC) add_residual16(x, v, res, kShift8 ? 8 : p.shift);
+              const uint32_t *sum = EPI == EPI_RES_NCHWC ? x : v;
+              const uint4 w = kShift8 ? pack16_shift8(sum) : pack16_shift(sum, p.shift);
+              if (mvalid) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(p.out) + og) = w;
             } else if constexpr (kRegroup) {
-              store_group16_regrouped(reinterpret_cast<uint32_t *>(p.out), xs, lane, vb, o_k, ok_k, o - obase + gstride);
+              store_group16_regrouped(reinterpret_cast<uint32_t *>(p.out), xs, lane, v, o_k, ok_k, og - obase);
             } else {
-              if (mvalid) finish_group16<EPI>(p, vb, o + gstride);
+              if (mvalid) finish_group16<EPI>(p, v, og);
             }
+          };
+          while (left > 0) {
+            if (left > 1) {
+              tmem_ld16(taddr + 16u, vb);
+              if constexpr (EPI == EPI_RES_NCHWC) {
+                if (mvalid) rb = *reinterpret_cast<const uint4 *>(p.residual + o + gstride);
+              }
+            }
+            group(va, ra, o);
+            tmem_ld_wait();
+            if (left > 2) {
+              tmem_ld16(taddr + 32u, va);
+              if constexpr (EPI == EPI_RES_NCHWC) {
+                if (mvalid) ra = *reinterpret_cast<const uint4 *>(p.residual + o + 2 * gstride);
+              }
+            }
+            if (left > 1) group(vb, rb, o + gstride);
+            tmem_ld_wait();
+            taddr += 32u;
+            o += 2 * gstride;
+            left -= 2;
           }
-          tmem_ld_wait();
-          taddr += 32u;
-          o += 2 * gstride;
-          left -= 2;
-        }
+        };
+        if (!epi_requantises(EPI) || p.shift == 8) drain_final(BoolTag<true>{});
+        else drain_final(BoolTag<false>{});
         drained = true;
       }
       if (!drained) {
