@@ -110,3 +110,38 @@ def test_requantising_drains_at_every_shift(U, n, c, h, co, shift):
                                   residual=None if res is None else dev(res))
         U.device_status()
         assert np.array_equal(got.cpu().numpy(), want)
+
+
+# grids smaller than the GPU: column blocks cut into narrow tiles (blocks of 144, 192, 208 and 256 columns, the last
+# one not full), with and without a split of the reduction, for every way the A operand arrives
+@pytest.mark.parametrize('m,n,k', [(1, 272, 256), (128, 3072, 768), (33, 208, 3072), (130, 1008, 1040), (500, 192, 4096), (300, 2064, 96)])
+def test_narrow_tiles_dense(U, m, n, k):
+    dense_case(U, m, n, k)
+    gemm_case(U, m, n, k)
+
+
+@pytest.mark.parametrize('n,c,h,w,co,k,s', [
+    (1, 256, 14, 14, 208, 3, 1),    # gather
+    (1, 512, 7, 7, 2048, 1, 1),     # gather, a short reduction for its width
+    (2, 192, 17, 17, 192, 7, 1),    # boxes, odd rows
+    (1, 288, 35, 35, 384, 3, 2),    # im2col copies
+    (1, 256, 28, 28, 272, 3, 2),    # pixel pairs
+])
+def test_narrow_tiles_conv(U, n, c, h, w, co, k, s):
+    from oracle import c_oracle
+    rng = np.random.default_rng(n + c + h + co)
+    p = k // 2
+    x = rng.integers(0, 256, (n, c // 16, h, w, 16), dtype=np.uint8)
+    wt = rng.integers(-128, 128, (co // 16, c // 16, k, k, 4, 16, 4), dtype=np.int8)
+    b = rng.integers(-2 ** 15, 2 ** 15, co, dtype=np.int32)
+    oh, ow = (h + 2 * p - k) // s + 1, (w + 2 * p - k) // s + 1
+    r = rng.integers(0, 256, (n, co // 16, oh, ow, 16), dtype=np.uint8)
+    xd, wd, bd = dev(x), dev(wt), dev(b)
+    for opt in ({}, {'bias': b}, {'bias': b, 'mul': 11}, {'bias': b, 'requant_shift': 10}, {'bias': b, 'requant_shift': 8, 'residual': r}):
+        want = c_oracle.conv2d_i8_ex(x, wt, (s, s), (p, p), **opt)
+        kw = {key: dev(v) if isinstance(v, np.ndarray) else v for key, v in opt.items()}
+        if 'requant_shift' in opt:
+            kw['out_dtype'] = 'uint8'
+        got = U.conv2d_NCHWc_int8(xd, wd, stride=s, padding=p, **kw)
+        U.device_status()
+        assert np.array_equal(got.cpu().numpy(), want), opt

@@ -124,6 +124,9 @@ struct IgemmParams {
   int k_stages;       // ceil(cols_padded / kc)
   int last_ksteps;    // MMA K-steps (2 columns each) in the last stage
   int stages;         // pipeline depth
+  // Narrow tiles: a packed weight block (b_row_bytes / 16 columns wide) is shared by b_sub tiles of bn columns each.
+  // A stage of such a tile is kc runs of bn * 16 bytes, b_row_bytes apart (b_sub = 1: one run).
+  int b_sub, b_row_bytes;
   int m_tiles, n_tiles;
   // convolution geometry (unused by A_DENSE)
   int H, W, Cc, OH, OW, KH, KW, sh, sw, ph, pw;
@@ -1180,7 +1183,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
     // ===================== B producer =====================
     // (p.inject: diagnostics.  The producer issues nothing, so no stage ever completes and the
     // bounded waits of the other roles run out: the path that reports UNIT_ERR_DEVICE_WAIT.)
-    if (lane == 0 && p.inject == 0) {
+    if (lane == 0 && p.inject == 0 && p.b_sub == 1) {
       uint32_t s = 0, ring_phase = 0;
       uint32_t lt = 0;
       bool alive = true;
@@ -1199,6 +1202,29 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           if (++s == (uint32_t)p.stages) { s = 0; ring_phase ^= 1u; }
         }
         trace_mark(p, lt, 2);
+      }
+    } else if (p.inject == 0 && p.b_sub > 1) {
+      // narrow tiles: one copy per K column of the stage, issued by as many lanes at once
+      const uint32_t run = (uint32_t)p.bn * 16u;
+      const size_t block_bytes = (size_t)p.kc * (size_t)p.b_row_bytes;
+      uint32_t s = 0, ring_phase = 0;
+      bool alive = true;
+      for (int tile = tile0; tile < total_tiles && alive; tile += tstep) {
+        const int n_tile = tile - (int)fast_div((uint32_t)tile, p.div_n_tiles) * p.n_tiles;
+        const int block = n_tile / p.b_sub;
+        const uint8_t *src = p.b + ((size_t)block * p.k_stages + ks_begin) * block_bytes + (size_t)(n_tile - block * p.b_sub) * run +
+                             (size_t)lane * p.b_row_bytes;
+        for (int ks = ks_begin; ks < ks_end; ++ks, src += block_bytes) {
+          if (!mbar_wait_warp(smem_u32(&ps->empty[s]), ring_phase ^ 1u, wc, kErrWaitEmpty)) {
+            alive = false;
+            break;
+          }
+          const uint32_t bar = smem_u32(&ps->full[s]);
+          if (lane == 0) mbar_arrive_expect_tx(bar, b_stage_bytes);
+          __syncwarp();
+          if (lane < p.kc) bulk_copy_g2s(smem_base + s * stage_bytes + a_stage_bytes + (uint32_t)lane * run, src, run, bar);
+          if (++s == (uint32_t)p.stages) { s = 0; ring_phase ^= 1u; }
+        }
       }
     }
   } else if (warp == kMmaWarp || (MT == 2 && warp == kMmaWarp2)) {

@@ -35,6 +35,7 @@ struct TileCfg {
   int bn = 0, kc = 0, cols = 0, cols_pad = 0, k_stages = 0, last_ksteps = 0, n_tiles = 0;
   size_t b_stage_bytes = 0;
   size_t a_stage_bytes = 0;  // window form: bytes of a stage's A part (0: kc columns x 128 rows per sub-tile)
+  int sub = 1;               // tiles per packed weight block (narrow tiles; bn and n_tiles are then the narrow ones)
 };
 
 constexpr size_t kSmemBudget = 200 * 1024;
@@ -676,6 +677,15 @@ static int max_active_clusters(const TileCfg &c, int ks) {
 // distributed shared memory (integer sums do not depend on the order, so the int8 results stay
 // bit-exact; the reference splits its reductions too: python/tensorizer/ops/gpu.py:83-87,134,
 // poc/tensorcore/gemm-prefetch.cu:29-64).  Returns 1 when the problem should not be split.
+static bool split_feasible(const TileCfg &c, int s) {
+  const int per = (c.k_stages + s - 1) / s;
+  if ((c.k_stages + per - 1) / per != s) return false;  // no CTA without stages
+  // the partial sums a CTA receives replace its operand ring: (S - 1) senders x owned groups x 128 rows x 64 bytes
+  size_t smem_bytes = 0;
+  const int stages = stages_for(c, 1, &smem_bytes);
+  const size_t ring = (size_t)stages * c.kc * 16 * (kTileM + c.bn);
+  return (size_t)(s - 1) * (((c.bn >> 4) + s - 1) / s) * kTileM * 64 <= ring;
+}
 static int choose_ksplit(const TileCfg &c, long long m_total, int sms, int table_ksplit = 0) {
   static const int forced_env = tuning_int("UNIT_B200_KSPLIT", -1);
   const int forced = table_ksplit > 0 ? table_ksplit : forced_env;  // a tile-table entry: 1 = never, n = at most n
@@ -693,14 +703,39 @@ static int choose_ksplit(const TileCfg &c, long long m_total, int sms, int table
   if (s < 2) return 1;
   const int per = (c.k_stages + s - 1) / s;
   s = (c.k_stages + per - 1) / per;          // no CTA without stages
-  if (s < 2) return 1;
-  // the partial sums a CTA receives replace its operand ring: (S - 1) senders x owned groups x 128 rows x 64 bytes
-  size_t smem_bytes = 0;
-  const int stages = stages_for(c, 1, &smem_bytes);
-  const size_t ring = (size_t)stages * c.kc * 16 * (kTileM + c.bn);
-  const size_t recv = (size_t)(s - 1) * (((c.bn >> 4) + s - 1) / s) * kTileM * 64;
-  return recv <= ring ? s : 1;
+  return s >= 2 && split_feasible(c, s) ? s : 1;
 }
+
+// ---- narrow tiles ----
+// A grid of fewer tiles than SMs is latency: one tile per CTA, and the tile's time is what its K loop, its drain and
+// the exchange of a split take.  Cutting the packed column blocks into narrower tiles (the packed form stays as it
+// is: a stage is then kc runs of bn * 16 bytes) gives more CTAs with shorter drains, a split of the reduction
+// shortens the K loop.  The estimate below is a least-squares fit to 860 measured (shape, sub, split) combinations
+// of 78 int8 and fp16 convolutions and products (relative error 6 %); over those shapes the times it picks sum to
+// 493 us, the best of each to 489, whole blocks with the split rule above to 601 (ResNet-50 at batch 1 in one
+// graph: 410 -> 354 us of kernels; dense 128x3072x768: 10.6 -> 8.5 us; fp16 3x3/2 128 at 56x56: 15.9 -> 8.4 us).
+// A tile-table entry's split limit holds here too.  Microseconds:
+//   fixed 1.7 + drain 2.2 per 256 columns + 1.7 per full GPU of CTAs (they share L2)
+//   + reduction columns of one CTA x the A operand's cost per 16-byte column (column_us)
+//   + split: 1.4 + 0.22 per peer + 3.6 per 256 columns sent
+static double tile_us(const TileCfg &t, long long m_tiles, int s, double per_col, int sms) {
+  const double width = t.bn / 256.0;
+  double us = 1.7 + 2.2 * width + 1.7 * (double)(m_tiles * t.n_tiles * s) / sms + per_col * t.cols_pad / s;
+  if (s > 1) us += 1.4 + 0.22 * (s - 1) + 3.6 * width * (s - 1) / s;
+  return us;
+}
+static double column_us(int amode, bool f16, bool pairs) {
+  switch (amode) {
+    case A_CONV_I8: return 0.148;
+    case A_CONV_F16: return 0.148;   // (the u8 gather's: the same loop)
+    case A_STEM_I8: return 0.148;
+    case A_DENSE: return 0.074;
+    case A_CONV_TMA: return f16 ? 0.095 : 0.086;
+    case A_DENSE_TMA: return 0.048;
+    default: return f16 ? 0.052 : (pairs ? 0.054 : 0.066);   // boxes
+  }
+}
+constexpr double kNarrowMargin = 0.92;  // estimated gains below 8 % are within the fit's error
 
 static FastDiv make_fast_div(uint32_t d);
 
@@ -720,6 +755,28 @@ static unsigned int *error_word_address() {
   return cached[dev];
 }
 
+static void set_tile(IgemmParams &p, const TileCfg &c) {
+  p.bn = c.bn;
+  p.kc = c.kc;
+  p.cols = c.cols;
+  p.k_stages = c.k_stages;
+  p.last_ksteps = c.last_ksteps;
+  p.n_tiles = c.n_tiles;
+  p.div_n_tiles = make_fast_div((uint32_t)c.n_tiles);
+  p.b_sub = c.sub;
+  p.b_row_bytes = c.sub * c.bn * 16;
+}
+
+// The tile shape with every packed column block cut into `sub` tiles.
+static TileCfg narrow_cfg(const TileCfg &c, int n_total, int sub) {
+  TileCfg t = c;
+  t.sub = sub;
+  t.bn = c.bn / sub;
+  t.n_tiles = (n_total + t.bn - 1) / t.bn;
+  t.b_stage_bytes = (size_t)t.kc * t.bn * 16;
+  return t;
+}
+
 // Fills the tile fields of the plan's parameters and picks the sub-tile count.  MAX_MT = 1 for
 // operand paths that only small problems reach (no two-sub-tile variant is compiled for them).
 template <int AMODE, int EPI, bool F16, int MAX_MT = 2>
@@ -728,13 +785,7 @@ static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = 
   pl.map_base = tmap_in == nullptr ? 0 : (pl.fold_n > 0 ? 2 : 1);
   if (tmap_in) memcpy(pl.map, tmap_in, sizeof(CUtensorMap));
   else memset(pl.map, 0, sizeof(pl.map));
-  p.bn = c.bn;
-  p.kc = c.kc;
-  p.cols = c.cols;
-  p.k_stages = c.k_stages;
-  p.last_ksteps = c.last_ksteps;
-  p.n_tiles = c.n_tiles;
-  p.div_n_tiles = make_fast_div((uint32_t)c.n_tiles);
+  set_tile(p, c);
   p.err = error_word_address();
   if (p.err == nullptr) return UNIT_ERR_LAUNCH;
   if (cudaGetDevice(&pl.device) != cudaSuccess) return UNIT_ERR_LAUNCH;
@@ -745,23 +796,41 @@ static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = 
     const int mt = (pl.table_mt == 1 || pl.table_mt == 2) ? pl.table_mt : choose_mt(c, p.m_total, sms, AMODE == A_CONV_TMA || F16);
     if (mt == 2) return prepare_mt<AMODE, EPI, F16, 2, false>(pl, c, sms, 1);
   }
-  if constexpr ((a_mode_uses_tma(AMODE) && AMODE != A_CONV_WIN) || AMODE == A_CONV_I8) {  // (the window form is used on full grids only;
-                                                                                        //  of the gathers, the u8 convolution's has a split-K form)
-    int ks = choose_ksplit(c, p.m_total, sms, pl.table_ksplit);
+  constexpr bool kSplits = (a_mode_uses_tma(AMODE) && AMODE != A_CONV_WIN) || AMODE == A_CONV_I8;  // (the window form is used on full
+                                                                                          // grids only; of the gathers, the u8 convolution's)
+  const long long mt1 = (p.m_total + kTileM - 1) / kTileM;
+  int ks = 1;
+  if constexpr (kSplits) {
+    ks = choose_ksplit(c, p.m_total, sms, pl.table_ksplit);
     // all clusters must be resident at once: a cluster needs its CTAs on SMs of one GPC, so fewer
     // clusters fit than SMs / size suggests (measured: 49 clusters of 3 ran in two rounds)
-    const long long tiles1 = (p.m_total + kTileM - 1) / kTileM * c.n_tiles;
-    while (ks > 1) {
-      const int per = (c.k_stages + ks - 1) / ks;
-      if ((c.k_stages + per - 1) / per == ks && tiles1 <= max_active_clusters<AMODE, EPI, F16>(c, ks)) break;
-      --ks;
-    }
-    if (ks > 1) return prepare_mt<AMODE, EPI, F16, 1, true>(pl, c, sms, ks);
-    // experiment builds: the split-K kernel with clusters of one CTA
-    static const int force1 = tuning_int("UNIT_B200_KSPLIT_ONE", 0);
-    if (force1 && (long long)((p.m_total + kTileM - 1) / kTileM) * c.n_tiles <= sms) return prepare_mt<AMODE, EPI, F16, 1, true>(pl, c, sms, 1);
+    while (ks > 1 && !(split_feasible(c, ks) && mt1 * c.n_tiles <= max_active_clusters<AMODE, EPI, F16>(c, ks))) --ks;
   }
-  return prepare_mt<AMODE, EPI, F16, 1, false>(pl, c, sms, 1);
+  TileCfg best = c;
+  if (mt1 * c.n_tiles <= sms) {
+    const double per_col = column_us(AMODE, F16, p.a_sw32 != 0);
+    double t_best = kNarrowMargin * tile_us(c, mt1, ks, per_col, sms);
+    for (int sub = 1; c.bn % (16 * sub) == 0 && c.bn / sub >= 16 && sub <= 16; ++sub) {
+      const TileCfg t = narrow_cfg(c, p.n_total, sub);
+      if (mt1 * t.n_tiles > sms) break;
+      const int s_max = !kSplits ? 1 : (pl.table_ksplit > 0 && pl.table_ksplit < 8 ? pl.table_ksplit : 8);
+      for (int s = 1; s <= s_max && mt1 * t.n_tiles * s <= sms; ++s) {
+        const double us = tile_us(t, mt1, s, per_col, sms);
+        if (us >= t_best) continue;
+        if constexpr (kSplits) {
+          if (s > 1 && !(split_feasible(t, s) && mt1 * t.n_tiles <= max_active_clusters<AMODE, EPI, F16>(t, s))) continue;
+        }
+        t_best = us;
+        best = t;
+        ks = s;
+      }
+    }
+    set_tile(p, best);
+  }
+  if constexpr (kSplits) {
+    if (ks > 1) return prepare_mt<AMODE, EPI, F16, 1, true>(pl, best, sms, ks);
+  }
+  return prepare_mt<AMODE, EPI, F16, 1, false>(pl, best, sms, 1);
 }
 
 // The int8 convolution's epilogue is chosen at run time: one instantiation per mode.

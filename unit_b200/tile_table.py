@@ -10,7 +10,8 @@ column block, the depth of a pipeline stage, sub-tiles per tile, the split-K lim
 * ``shape_corpus.json``  the int8 NCHW16c convolution shapes of the reference's ``cpu-shapes.log``
   (made by ``python -m unit_b200.tile_table corpus <cpu-shapes.log>``); shapes only, no data;
 * ``tile_table.json``    entries found by ``python -m unit_b200.tune`` on a B200; loaded and handed
-  to the library on first use of an operator (absent file: heuristics only).
+  to the library on first use of an operator (absent file: heuristics only).  Sizes of at most one
+  128-row tile per SM carry no entry: there the library's own estimate also picks the tile's width.
 """
 from __future__ import annotations
 
