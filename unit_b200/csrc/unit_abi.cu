@@ -634,17 +634,15 @@ static int prepare_mt(PlanImpl &pl, const TileCfg &c, int sms, int ksplit) {
 }
 
 // How many clusters of `ks` CTAs of the split-K kernel the current device holds at once (cached per
-// kernel variant, size and shared-memory request).
+// kernel variant and cluster size; the answer is for the largest shared-memory request).
 template <int AMODE, int EPI, bool F16>
-static int max_active_clusters(const TileCfg &c, int ks) {
+static int max_active_clusters(int ks) {
   static std::mutex mu;
-  static int cached[64][9][kMaxStages + 1] = {};
-  size_t smem_bytes = 0;
-  const int stages = stages_for(c, 1, &smem_bytes);
+  static int cached[64][9] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || ks < 2 || ks > 8) return 0;
   std::lock_guard<std::mutex> lock(mu);
-  int &slot = cached[dev][ks][stages];
+  int &slot = cached[dev][ks];
   if (slot == 0) {
     auto kern = igemm_kernel<AMODE, EPI, F16, 1, true>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
@@ -804,7 +802,7 @@ static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = 
     ks = choose_ksplit(c, p.m_total, sms, pl.table_ksplit);
     // all clusters must be resident at once: a cluster needs its CTAs on SMs of one GPC, so fewer
     // clusters fit than SMs / size suggests (measured: 49 clusters of 3 ran in two rounds)
-    while (ks > 1 && !(split_feasible(c, ks) && mt1 * c.n_tiles <= max_active_clusters<AMODE, EPI, F16>(c, ks))) --ks;
+    while (ks > 1 && !(split_feasible(c, ks) && mt1 * c.n_tiles <= max_active_clusters<AMODE, EPI, F16>(ks))) --ks;
   }
   TileCfg best = c;
   if (mt1 * c.n_tiles <= sms) {
@@ -818,7 +816,7 @@ static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = 
         const double us = tile_us(t, mt1, s, per_col, sms);
         if (us >= t_best) continue;
         if constexpr (kSplits) {
-          if (s > 1 && !(split_feasible(t, s) && mt1 * t.n_tiles <= max_active_clusters<AMODE, EPI, F16>(t, s))) continue;
+          if (s > 1 && !(split_feasible(t, s) && mt1 * t.n_tiles <= max_active_clusters<AMODE, EPI, F16>(s))) continue;
         }
         t_best = us;
         best = t;
