@@ -67,6 +67,22 @@ def test_gemm_reductions_that_end_inside_a_stage(U, m, n, k):
     gemm_case(U, m, n, k)
 
 
+# Reductions below one 128-byte stage arrive as 16-byte columns, two per K step.  With an odd number of columns the
+# last step's second one exists in no matrix: it must read as zero whatever an earlier kernel left in shared memory
+# (here: bytes that are NaN in fp16).  One and two sub-tiles per tile, a ragged last row block; even counts beside odd.
+@pytest.mark.parametrize('m,n,k', [(8200, 64, 8), (40007, 64, 8), (2800, 272, 24), (40007, 32, 24), (1700, 48, 40), (20011, 128, 40),
+                                   (8200, 64, 16), (2050, 528, 32), (1501, 64, 48)])
+def test_gemm_column_copies_after_another_kernel(U, m, n, k):
+    from unit_b200 import _lib
+    # (the packed form shows which one runs: a 128-byte stage holds 8 columns of 16 bytes)
+    assert m * k * 2 >= 131072 and _lib.lib().unit_packed_weights_bytes_gemm_f16(n, k) < n * 128
+    a = torch.full((3000, 4096), 0x7c, dtype=torch.uint8, device='cuda')
+    wq = U.pack_dense_weights_int8(torch.ones((16, 1024, 16, 4), dtype=torch.int8, device='cuda'))
+    for _ in range(3):
+        U.dense_dotprod(a, wq)
+        gemm_case(U, m, n, k)
+
+
 # (batch, chunks, depth, h, w, c_out, kernel, padding): one and two sub-tiles, padding in no and in every dimension,
 # kernels that are flat in one dimension, slices smaller than a tile, a column block that is not full
 @pytest.mark.parametrize('n,c,d,h,w,co,k,p', [

@@ -1131,6 +1131,9 @@ __global__ void __launch_bounds__(kNumThreads, 1)
         const uint32_t bar = smem_u32(&ps->full[s]);
         int real = p.cols - ks * p.kc;  // columns of this stage that exist (the rest only meets zero weights)
         real = real < 0 ? 0 : (real > p.kc ? p.kc : real);
+        // (in fp16 a zero weight does not cancel what shared memory happens to hold: NaN and infinities stay.  The K
+        // step of an odd last column therefore gets the column after it too, which lies outside the map: zeros)
+        if (F16 && AMODE == A_DENSE_TMA) real = (real + 1) & ~1;
         if (AMODE == A_DENSE_TMA && p.a_sw128 != 0) {
           // one copy = 128 rows x 128 bytes of K (8 columns) of one sub-tile, written swizzled
           const int atoms = p.kc >> 3;
