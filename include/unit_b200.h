@@ -250,6 +250,14 @@ int unit_conv2d_int8_nchwc(const unit_conv_desc *desc, const void *d_x, const vo
 int unit_conv2d_plan_int8(const unit_conv_desc *desc, const void *d_x, const void *d_packed_w,
                           const unit_epilogue *epilogue, void *d_out, void *d_workspace,
                           size_t workspace_bytes, unit_conv_plan *plan);
+/* The same for a launch that will run beside others (parallel branches of a CUDA graph, several streams): tile
+ * width and split of small grids are chosen for the SM time they take, not for the launch's own latency.  Same
+ * results. */
+int unit_conv2d_plan_int8_shared(const unit_conv_desc *desc, const void *d_x, const void *d_packed_w,
+                                 const unit_epilogue *epilogue, void *d_out, void *d_workspace,
+                                 size_t workspace_bytes, unit_conv_plan *plan);
+/* Thread blocks the plan's contraction launches, at most one per SM (negative: a status code). */
+int unit_plan_ctas(const unit_conv_plan *plan);
 int unit_conv2d_run(const unit_conv_plan *plan, void *stream);
 /* Points a plan at other buffers of the same shapes (the reference's built module is likewise called with
  * new arrays each time): tile selection and tensor map stay, only addresses change.  d_x is the activations

@@ -161,3 +161,24 @@ def test_narrow_tiles_conv(U, n, c, h, w, co, k, s):
         got = U.conv2d_NCHWc_int8(xd, wd, stride=s, padding=p, **kw)
         U.device_status()
         assert np.array_equal(got.cpu().numpy(), want), opt
+
+
+@pytest.mark.parametrize('batch', [1, 16])
+def test_shared_plans_take_fewer_blocks_and_give_the_same_results(U, batch):
+    """Launches that run beside others: SM time counts, so a small grid is cut less than for its own latency."""
+    from unit_b200 import resnet50 as R
+    alone, shared = {}, {}
+    for i, l in enumerate(R.LAYERS):
+        if l.c_block != 16:
+            continue
+        x, w, b = (dev(a) for a in R.make_layer_inputs(l, i, batch))
+        pw = U.pack_conv_weights_int8(w, l.stride, l.pad)
+        opt = dict(stride=l.stride, padding=l.pad, bias=b, out_dtype='uint8')
+        plans = [U.conv2d_NCHWc_int8_plan(x, pw, shared=s, **opt) for s in (False, True)]
+        assert torch.equal(plans[0].run(), plans[1].run()), l.name
+        alone[l.name], shared[l.name] = plans[0].ctas * l.count, plans[1].ctas * l.count
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        assert 1 <= plans[1].ctas <= plans[0].ctas <= sms, l.name
+    U.device_status()
+    # per layer the time of a block grows as their number falls, but by less than the number does
+    assert sum(shared.values()) < 0.9 * sum(alone.values()), (alone, shared)

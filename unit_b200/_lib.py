@@ -85,6 +85,8 @@ SIGNATURES = {
     'unit_conv2d_u8s8_requant_nchwc': (_ci, [_dp, _vp, _vp, _vp, _ci, _vp, _vp, _sz, _vp]),
     'unit_conv2d_int8_nchwc': (_ci, [_dp, _vp, _vp, _ep, _vp, _vp, _sz, _vp]),
     'unit_conv2d_plan_int8': (_ci, [_dp, _vp, _vp, _ep, _vp, _vp, _sz, _pp]),
+    'unit_conv2d_plan_int8_shared': (_ci, [_dp, _vp, _vp, _ep, _vp, _vp, _sz, _pp]),
+    'unit_plan_ctas': (_ci, [_pp]),
     'unit_conv2d_run': (_ci, [_pp, _vp]),
     'unit_plan_rebind': (_ci, [_pp, _vp, _vp, _vp, _vp, _vp]),
     'unit_packed_weights_bytes_conv3d_i8': (_sz, [_d3]),

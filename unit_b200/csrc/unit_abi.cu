@@ -589,6 +589,7 @@ struct PlanImpl {
   uint32_t grid, smem_bytes;
   uint32_t cluster;                  // > 1: thread-block cluster size (split-K)
   int32_t table_mt, table_ksplit;    // from the tile table: 0 = heuristics (ksplit 1 = do not split)
+  int32_t shared;                    // the launch runs beside others: tiles are chosen for the SM time they take
   int32_t fold_n, fold_h2, fold_w2;  // fold_n > 0: the stem's 2 x 2 fold into scratch runs first
   const void *fold_src;
   void *fold_dst;
@@ -713,12 +714,21 @@ static int choose_ksplit(const TileCfg &c, long long m_total, int sms, int table
 // 493 us, the best of each to 489, whole blocks with the split rule above to 601 (ResNet-50 at batch 1 in one
 // graph: 410 -> 354 us of kernels; dense 128x3072x768: 10.6 -> 8.5 us; fp16 3x3/2 128 at 56x56: 15.9 -> 8.4 us).
 // A tile-table entry's split limit holds here too.  Microseconds:
-//   fixed 1.7 + drain 2.2 per 256 columns + 1.7 per full GPU of CTAs (they share L2)
+//   fixed 1.7 + drain 2.2 per 256 columns + a price per full GPU of CTAs
 //   + reduction columns of one CTA x the A operand's cost per 16-byte column (column_us)
 //   + split: 1.4 + 0.22 per peer + 3.6 per 256 columns sent
-static double tile_us(const TileCfg &t, long long m_tiles, int s, double per_col, int sms) {
+// What a CTA costs depends on what else the GPU has to do.  A launch that has it to itself pays 1.7 per full GPU of
+// CTAs (they share L2).  Launches that run side by side (parallel graph branches, several streams) compete for SMs,
+// and a tile cut in two is two drains and two A operands: there the price is 15, and whole blocks have no margin.
+// ResNet-50's 54 launches in six branches and as one chain, ms, at batch 1 / 4 / 8 / 16 / 32:
+//   price 1.7: 0.111 / 0.177 / 0.259 / 0.368 / 0.466, chain 0.364 / 0.359 / 0.372 / 0.431 / 0.511
+//   price 15:  0.090 / 0.148 / 0.208 / 0.287 / 0.407, chain 0.381 / 0.378 / 0.398 / 0.445 / 0.525
+//   whole blocks with the split rule above: 0.092 / 0.173 / 0.284 / 0.384 / 0.466, chain 0.426 / 0.403 / 0.417 / 0.448 / 0.513
+// Prices between (2.5 to 10) lie between on both counts, so the caller says which one counts.
+constexpr double kCtaPriceAlone = 1.7, kCtaPriceShared = 15.0;
+static double tile_us(const TileCfg &t, long long m_tiles, int s, double per_col, int sms, double cta_price) {
   const double width = t.bn / 256.0;
-  double us = 1.7 + 2.2 * width + 1.7 * (double)(m_tiles * t.n_tiles * s) / sms + per_col * t.cols_pad / s;
+  double us = 1.7 + 2.2 * width + cta_price * (double)(m_tiles * t.n_tiles * s) / sms + per_col * t.cols_pad / s;
   if (s > 1) us += 1.4 + 0.22 * (s - 1) + 3.6 * width * (s - 1) / s;
   return us;
 }
@@ -807,13 +817,14 @@ static int prepare(PlanImpl &pl, const TileCfg &c, const CUtensorMap *tmap_in = 
   TileCfg best = c;
   if (mt1 * c.n_tiles <= sms) {
     const double per_col = column_us(AMODE, F16, p.a_sw32 != 0);
-    double t_best = kNarrowMargin * tile_us(c, mt1, ks, per_col, sms);
+    const double price = pl.shared ? kCtaPriceShared : kCtaPriceAlone;
+    double t_best = (pl.shared ? 1.0 : kNarrowMargin) * tile_us(c, mt1, ks, per_col, sms, price);
     for (int sub = 1; c.bn % (16 * sub) == 0 && c.bn / sub >= 16 && sub <= 16; ++sub) {
       const TileCfg t = narrow_cfg(c, p.n_total, sub);
       if (mt1 * t.n_tiles > sms) break;
       const int s_max = !kSplits ? 1 : (pl.table_ksplit > 0 && pl.table_ksplit < 8 ? pl.table_ksplit : 8);
       for (int s = 1; s <= s_max && mt1 * t.n_tiles * s <= sms; ++s) {
-        const double us = tile_us(t, mt1, s, per_col, sms);
+        const double us = tile_us(t, mt1, s, per_col, sms, price);
         if (us >= t_best) continue;
         if constexpr (kSplits) {
           if (s > 1 && !(split_feasible(t, s) && mt1 * t.n_tiles <= max_active_clusters<AMODE, EPI, F16>(s))) continue;
@@ -1201,7 +1212,7 @@ struct EpilogueArgs {
 };
 
 static int plan_conv_i8(PlanImpl &pl, const unit_conv_desc *d, const void *x, const void *pw, const EpilogueArgs &e,
-                        void *out, void *workspace, size_t workspace_bytes) {
+                        void *out, void *workspace, size_t workspace_bytes, bool shared = false) {
   int rc = check_conv(d, false);
   if (rc) return rc;
   if (!x || !pw || !out) return UNIT_ERR_NULL;
@@ -1214,6 +1225,7 @@ static int plan_conv_i8(PlanImpl &pl, const unit_conv_desc *d, const void *x, co
   const int epi = e.out_u8 ? (e.residual ? EPI_RES_NCHWC : EPI_REQ_NCHWC) : (e.mul != 1 ? EPI_MUL_NCHWC : EPI_RAW_NCHWC);
   const TileCfg c = conv_cfg_i8(d);
   pl = PlanImpl{};
+  pl.shared = shared ? 1 : 0;
   {
     unit_tile_entry te;
     if (d->c_block == 16 && tile_lookup(d, &te)) {
@@ -1819,14 +1831,30 @@ static int export_plan(int rc, const PlanImpl &pl, unit_conv_plan *plan) {
   return UNIT_OK;
 }
 
-int unit_conv2d_plan_int8(const unit_conv_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out,
-                          void *workspace, size_t workspace_bytes, unit_conv_plan *plan) {
+static int plan_int8(const unit_conv_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out, void *workspace,
+                     size_t workspace_bytes, bool shared, unit_conv_plan *plan) {
   if (!plan) return UNIT_ERR_NULL;
   EpilogueArgs e;
   int rc = epilogue_from(epi, &e);
   if (rc) return rc;
   PlanImpl pl;
-  return export_plan(plan_conv_i8(pl, d, x, pw, e, out, workspace, workspace_bytes), pl, plan);
+  return export_plan(plan_conv_i8(pl, d, x, pw, e, out, workspace, workspace_bytes, shared), pl, plan);
+}
+
+int unit_conv2d_plan_int8(const unit_conv_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out,
+                          void *workspace, size_t workspace_bytes, unit_conv_plan *plan) {
+  return plan_int8(d, x, pw, epi, out, workspace, workspace_bytes, false, plan);
+}
+
+int unit_conv2d_plan_int8_shared(const unit_conv_desc *d, const void *x, const void *pw, const unit_epilogue *epi, void *out,
+                                 void *workspace, size_t workspace_bytes, unit_conv_plan *plan) {
+  return plan_int8(d, x, pw, epi, out, workspace, workspace_bytes, true, plan);
+}
+
+int unit_plan_ctas(const unit_conv_plan *plan) {
+  if (!plan) return UNIT_ERR_NULL;
+  const PlanImpl *pl = reinterpret_cast<const PlanImpl *>(plan);
+  return pl->magic == kPlanMagic ? (int)pl->grid : UNIT_ERR_SHAPE;
 }
 
 int unit_plan_rebind(unit_conv_plan *plan, const void *x, const int32_t *bias, const void *residual, void *out, void *workspace) {

@@ -282,6 +282,11 @@ class ConvPlan:
         self._keep = keep
         self._run = _lib.host().Runner(ctypes.addressof(plan), out).run
 
+    @property
+    def ctas(self) -> int:
+        """Thread blocks of the contraction, at most one per SM."""
+        return int(_lib.lib().unit_plan_ctas(ctypes.byref(self._plan)))
+
     def run(self) -> torch.Tensor:
         r = self._run()
         if type(r) is int:
@@ -401,9 +406,12 @@ def conv2d_NCHWc_int8_plan(data: torch.Tensor, kernel, stride: IntPair = 1, padd
                            dilation: IntPair = 1, layout: str = 'NCHW4c', out_layout: str = 'NCHW16c',
                            out_dtype: str = 'int32', *, bias: Optional[torch.Tensor] = None,
                            requant_shift: Optional[int] = None, mul: int = 1,
-                           residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> ConvPlan:
+                           residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+                           shared: bool = False) -> ConvPlan:
     """Same arguments as ``conv2d_NCHWc_int8`` (CUDA tensors only); returns a ``ConvPlan`` whose
-    ``run()`` repeats the convolution on these buffers."""
+    ``run()`` repeats the convolution on these buffers.  ``shared``: the launch will run beside others
+    (parallel branches of a CUDA graph, several streams), so the SM time it takes counts and not its
+    own latency; small grids then take fewer thread blocks.  Same results."""
     if not data.is_cuda:
         raise ValueError('a plan is bound to device buffers: pass CUDA tensors')
     L, d, tensors, epi, out_t, ws, ws_bytes, _host, n = _conv_int8_prepare(
@@ -413,8 +421,9 @@ def conv2d_NCHWc_int8_plan(data: torch.Tensor, kernel, stride: IntPair = 1, padd
     x, pw = tensors[0], tensors[1]
     plan = _CPlan()
     with torch.cuda.device(x.device):
-        check(L.unit_conv2d_plan_int8(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
-                                      ws_bytes, ctypes.byref(plan)), 'unit_conv2d_plan_int8')
+        make = L.unit_conv2d_plan_int8_shared if shared else L.unit_conv2d_plan_int8
+        check(make(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
+                   ws_bytes, ctypes.byref(plan)), 'unit_conv2d_plan_int8')
     return ConvPlan(plan, out_t, tensors + (ws,))
 
 
