@@ -85,3 +85,62 @@ def test_products_and_fp16_convolutions_read_their_own_buffers(U, m):
         bound = 288 * 2.0 ** -24 * torch.nn.functional.conv2d(xc.abs(), wc.abs(), padding=1) + 1e-30
         assert bool(((got - want).abs() <= bound).all())
     U.device_status()
+
+
+class Calls:
+    """Counts the calls that take the operator's own checks instead of a kept plan."""
+
+    def __init__(self, monkeypatch):
+        from unit_b200 import ops
+        self.n = 0
+        prepare = ops._conv_int8_prepare
+
+        def counted(*a):
+            self.n += 1
+            return prepare(*a)
+        monkeypatch.setattr(ops, '_conv_int8_prepare', counted)
+
+
+def conv_case(U, case, g):
+    w = torch.randint(-128, 128, case['w'], dtype=torch.int8, device='cuda', generator=g)
+    kw = dict(stride=case['stride'], padding=case['padding'])
+    return U.pack_conv_weights_int8(w, **kw), kw
+
+
+@pytest.mark.parametrize('case', CONV)
+def test_any_number_of_named_outputs_and_inputs(U, case, monkeypatch):
+    g = gen(7)
+    pw, kw = conv_case(U, case, g)
+    xs = [u8(case['x'], g) for _ in range(3)]
+    want = [U.conv2d_NCHWc_int8_plan(x, pw, **kw).run() for x in xs]
+    ring = [torch.empty_like(want[0]) for _ in range(40)]
+    calls = Calls(monkeypatch)
+    for _ in range(2):
+        for i, out in enumerate(ring):
+            out.zero_()
+            assert U.conv2d_NCHWc_int8(xs[i % 3], pw, out=out, **kw) is out
+        for i, out in enumerate(ring):
+            assert torch.equal(out, want[i % 3])
+    assert calls.n == 1
+    U.device_status()
+
+
+@pytest.mark.parametrize('case', CONV)
+@pytest.mark.parametrize('named', [False, True])
+def test_streams_that_take_turns(U, case, named, monkeypatch):
+    """One plan serves every stream; the folded stem's scratch is each stream's own."""
+    g = gen(8)
+    pw, kw = conv_case(U, case, g)
+    x = [u8(case['x'], g) for _ in range(2)]
+    want = [U.conv2d_NCHWc_int8_plan(t, pw, **kw).run() for t in x]
+    out = [torch.empty_like(t) for t in want]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    calls = Calls(monkeypatch)
+    for _ in range(6):
+        for s in (0, 1):
+            with torch.cuda.stream(streams[s]):
+                got = U.conv2d_NCHWc_int8(x[s], pw, out=out[s] if named else None, **kw)
+                assert torch.equal(got, want[s])
+    assert calls.n == 2     # each stream's first call (it waits for the weights and gets its scratch)
+    U.device_status()

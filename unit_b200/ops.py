@@ -294,17 +294,6 @@ class ConvPlan:
         return r
 
 
-class _NamedLaunches:
-    """The prepared launches of calls that named their output buffer: the launchers keep them, one per
-    set of buffers."""
-
-    def __len__(self) -> int:
-        return _lib.host().bound_count()
-
-
-_PLAN_CACHE = _NamedLaunches()
-
-
 def _conv_int8_prepare(data, kernel, stride, padding, dilation, out_layout, out_dtype, bias, requant_shift, mul,
                        residual, out):
     """Shared front end of ``conv2d_NCHWc_int8`` and ``conv2d_NCHWc_int8_plan``: checks the layout
