@@ -144,3 +144,25 @@ def test_streams_that_take_turns(U, case, named, monkeypatch):
                 assert torch.equal(got, want[s])
     assert calls.n == 2     # each stream's first call (it waits for the weights and gets its scratch)
     U.device_status()
+
+
+def test_an_allocation_that_fails_is_torch_s_out_of_memory_error(U):
+    """On repeated calls as on the first, so that a caller can free memory and try again."""
+    g = gen(9)
+    pw, kw = conv_case(U, dict(w=(4, 4, 3, 3, 4, 16, 4), stride=1, padding=1), g)
+    x = u8((64, 4, 56, 56, 16), g)
+    nchw = u8((64, 64, 56, 56), g)
+    runs = [lambda: U.conv2d_NCHWc_int8(x, pw, **kw), lambda: U.pack_data_nchwc(nchw), lambda: U.unpack_data_nchwc(x)]
+    want = [f().cpu() for f in runs]
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 2 ** 20) / total)
+    try:
+        for f in runs:
+            with pytest.raises(torch.OutOfMemoryError):
+                f()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for f, t in zip(runs, want):
+        assert torch.equal(f().cpu(), t)
+    U.device_status()

@@ -19,6 +19,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstring>
@@ -91,6 +92,13 @@ struct Launcher {
   std::vector<cudaStream_t> *streams;               // streams that have waited for the packed weights
   std::vector<std::shared_ptr<Entry>> *entries;   // (a call keeps its entry while others evict)
 };
+
+// The current C++ exception as the Python exception that torch gives it: a failed allocation is a
+// torch.OutOfMemoryError here as it is in the operators' own checks.
+PyObject *raise_in_python() {
+  torch::translate_exception_to_python(std::current_exception());
+  return nullptr;
+}
 
 bool get_int(PyObject *o, int64_t *v) {
   if (!PyLong_CheckExact(o)) return false;
@@ -257,9 +265,8 @@ PyObject *launcher_call(Launcher *self, PyObject *const *args, Py_ssize_t nargs)
     const int rc = launch(e->plan, st);
     if (rc) return PyLong_FromLong(rc);
     return named ? Py_NewRef(a[kArgOut]) : THPVariable_Wrap(std::move(out));
-  } catch (const std::exception &ex) {
-    PyErr_SetString(PyExc_RuntimeError, ex.what());
-    return nullptr;
+  } catch (...) {
+    return raise_in_python();
   }
 }
 
@@ -302,9 +309,8 @@ PyObject *launcher_add(Launcher *self, PyObject *const *args, Py_ssize_t nargs) 
     if (es.size() >= kMaxEntries) es.erase(es.begin());
     es.push_back(std::move(fresh));
     Py_RETURN_NONE;
-  } catch (const std::exception &ex) {
-    PyErr_SetString(PyExc_RuntimeError, ex.what());
-    return nullptr;
+  } catch (...) {
+    return raise_in_python();
   }
 }
 
@@ -315,7 +321,11 @@ PyObject *launcher_add_stream(Launcher *self, PyObject *o) {
     PyErr_SetString(PyExc_TypeError, "a stream handle is an int");
     return nullptr;
   }
-  self->streams->push_back(reinterpret_cast<cudaStream_t>(v));
+  try {
+    self->streams->push_back(reinterpret_cast<cudaStream_t>(v));
+  } catch (...) {
+    return raise_in_python();
+  }
   Py_RETURN_NONE;
 }
 
@@ -325,8 +335,13 @@ PyObject *launcher_new(PyTypeObject *type, PyObject *args, PyObject *) {
   Launcher *self = reinterpret_cast<Launcher *>(type->tp_alloc(type, 0));
   if (!self) return nullptr;
   self->device = device;
-  self->streams = new std::vector<cudaStream_t>();
-  self->entries = new std::vector<std::shared_ptr<Entry>>();
+  try {   // (the object's memory starts as zeros, so a half-made one can be dropped)
+    self->streams = new std::vector<cudaStream_t>();
+    self->entries = new std::vector<std::shared_ptr<Entry>>();
+  } catch (...) {
+    Py_DECREF(self);
+    return raise_in_python();
+  }
   return reinterpret_cast<PyObject *>(self);
 }
 void launcher_dealloc(Launcher *self) {
@@ -370,9 +385,8 @@ PyObject *runner_run(Runner *self, PyObject *) {
     rc = g_run(&self->plan, st);
     Py_END_ALLOW_THREADS
     return rc ? PyLong_FromLong(rc) : Py_NewRef(self->out);
-  } catch (const std::exception &ex) {
-    PyErr_SetString(PyExc_RuntimeError, ex.what());
-    return nullptr;
+  } catch (...) {
+    return raise_in_python();
   }
 }
 PyMethodDef runner_methods[] = {{"run", (PyCFunction)runner_run, METH_NOARGS, "launch the plan on the current stream"},
@@ -410,9 +424,8 @@ PyObject *layout_call(LayoutFn fn, PyObject *const *args, Py_ssize_t nargs, bool
     rc = fn(src, dst, (int32_t)n, (int32_t)c, (int32_t)h, (int32_t)w, (int32_t)cb, eb, st);
     Py_END_ALLOW_THREADS
     return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(out));
-  } catch (const std::exception &ex) {
-    PyErr_SetString(PyExc_RuntimeError, ex.what());
-    return nullptr;
+  } catch (...) {
+    return raise_in_python();
   }
 }
 PyObject *host_pack(PyObject *, PyObject *const *args, Py_ssize_t n) { return layout_call(g_pack, args, n, true); }
