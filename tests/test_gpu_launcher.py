@@ -166,3 +166,28 @@ def test_an_allocation_that_fails_is_torch_s_out_of_memory_error(U):
     for f, t in zip(runs, want):
         assert torch.equal(f().cpu(), t)
     U.device_status()
+
+
+def test_only_calls_with_packed_weights_pay_for_a_launcher(U):
+    """Packing makes none, nor does a call that packs raw weights itself (its next call cannot use it)."""
+    from unit_b200 import ops
+    g = gen(10)
+    w8 = torch.randint(-128, 128, (4, 4, 3, 3, 4, 16, 4), dtype=torch.int8, device='cuda', generator=g)
+    wd = torch.randint(-128, 128, (4, 256, 16, 4), dtype=torch.int8, device='cuda', generator=g)
+    wf = torch.randn((2, 2, 3, 3, 16, 16), device='cuda', generator=g).half()
+    bg = torch.randn((512, 64), device='cuda', generator=g).half()
+    x8, xd = u8((2, 4, 20, 20, 16), g), u8((70, 1024), g)
+    xf, xg = torch.randn((2, 2, 12, 12, 16), device='cuda', generator=g).half(), torch.randn((70, 512), device='cuda', generator=g).half()
+    for pack, w, call in ((lambda w: U.pack_conv_weights_int8(w, 1, 1), w8, lambda w: U.conv2d_NCHWc_int8(x8, w, padding=1)),
+                          (U.pack_dense_weights_int8, wd, lambda w: U.dense_dotprod(xd, w)),
+                          (U.pack_conv_weights_f16, wf, lambda w: U.conv2d_NCHW16c_OHWI16o(xf, w, 1, 1, padding=1)),
+                          (U.pack_gemm_weights_f16, bg, lambda w: U.gemm_f16f32(xg, w))):
+        raw = [call(w) for _ in range(2)]
+        pw = pack(w)                                  # (the tensor's packed copy is cached: the one these calls used)
+        assert pw._launcher is None
+        n = ops.launch_count()
+        packed = [call(pw) for _ in range(3)]
+        assert ops.launch_count() == n + 3 and pw._launcher is not None
+        for t in raw + packed:
+            assert torch.equal(t, raw[0])
+    U.device_status()

@@ -270,44 +270,49 @@ PyObject *launcher_call(Launcher *self, PyObject *const *args, Py_ssize_t nargs)
   }
 }
 
-// add(plan_address, result, workspace_address, c_out, op, data, bias, residual, out, options...): keeps the
-// plan that the operator just made and ran for this call (`result` is the tensor it wrote)
-PyObject *launcher_add(Launcher *self, PyObject *const *args, Py_ssize_t nargs) {
+// Keeps the plan of the call `a` (its operator number and arguments); `result` is the tensor it writes.
+void keep(Launcher *self, int64_t plan_addr, PyObject *result_obj, void *workspace, int64_t c_out, int64_t op, PyObject *const *a,
+          Py_ssize_t n, cudaStream_t st) {
+  const at::Tensor *x = cuda_tensor(a[kArgData], self->device);
+  const at::Tensor *result = cuda_tensor(result_obj, self->device);
+  Key k;
+  if (!x || !result || c10::cuda::current_device() != self->device || !make_key(k, op, a, n, *x)) return;
+  if (const std::shared_ptr<Entry> e = find_entry(self, k)) {  // known, but not on this stream
+    if (e->needs_scratch && workspace) e->set_scratch(st, workspace);
+    return;
+  }
+  auto fresh = std::make_shared<Entry>();
+  fresh->key = k;
+  fresh->c_out = c_out;
+  fresh->out_sizes = result->sizes().vec();
+  fresh->out_type = result->scalar_type();
+  Ptrs p;
+  p.x = x->data_ptr();
+  p.out = result->data_ptr();
+  p.workspace = workspace;
+  if (!optional_ptrs(*fresh, a, self->device, p)) return;
+  memcpy(&fresh->plan, reinterpret_cast<const void *>(plan_addr), sizeof(unit_conv_plan));
+  fresh->at = p;
+  fresh->needs_scratch = workspace != nullptr;
+  if (workspace) fresh->set_scratch(st, workspace);
+  auto &es = *self->entries;
+  if (es.size() >= kMaxEntries) es.erase(es.begin());
+  es.push_back(std::move(fresh));
+}
+
+// run(plan_address, result, workspace_address, c_out, op, data, bias, residual, out, options...): launches the plan
+// that the operator made for this call and keeps it (`result` is the tensor it writes) -> None or an int
+PyObject *launcher_run(Launcher *self, PyObject *const *args, Py_ssize_t nargs) {
   int64_t plan_addr, ws_addr, c_out, op;
   if (nargs < 9 || !get_int(args[0], &plan_addr) || !get_int(args[2], &ws_addr) || !get_int(args[3], &c_out) || !get_int(args[4], &op)) {
-    PyErr_SetString(PyExc_TypeError, "add(plan, result, workspace, c_out, op, data, bias, residual, out, options...)");
+    PyErr_SetString(PyExc_TypeError, "run(plan, result, workspace, c_out, op, data, bias, residual, out, options...)");
     return nullptr;
   }
-  PyObject *const *a = args + 5;
-  const Py_ssize_t n = nargs - 5;
   try {
-    const at::Tensor *x = cuda_tensor(a[kArgData], self->device);
-    const at::Tensor *result = cuda_tensor(args[1], self->device);
-    Key k;
-    if (!x || !result || c10::cuda::current_device() != self->device || !make_key(k, op, a, n, *x)) Py_RETURN_NONE;
-    const cudaStream_t st = c10::cuda::getCurrentCUDAStream(self->device).stream();
-    void *workspace = reinterpret_cast<void *>(ws_addr);
-    if (const std::shared_ptr<Entry> e = find_entry(self, k)) {  // known, but not on this stream
-      if (e->needs_scratch && workspace) e->set_scratch(st, workspace);
-      Py_RETURN_NONE;
-    }
-    auto fresh = std::make_shared<Entry>();
-    fresh->key = k;
-    fresh->c_out = c_out;
-    fresh->out_sizes = result->sizes().vec();
-    fresh->out_type = result->scalar_type();
-    Ptrs p;
-    p.x = x->data_ptr();
-    p.out = result->data_ptr();
-    p.workspace = workspace;
-    if (!optional_ptrs(*fresh, a, self->device, p)) Py_RETURN_NONE;
-    memcpy(&fresh->plan, reinterpret_cast<const void *>(plan_addr), sizeof(unit_conv_plan));
-    fresh->at = p;
-    fresh->needs_scratch = workspace != nullptr;
-    if (workspace) fresh->set_scratch(st, workspace);
-    auto &es = *self->entries;
-    if (es.size() >= kMaxEntries) es.erase(es.begin());
-    es.push_back(std::move(fresh));
+    const cudaStream_t st = c10::cuda::getCurrentCUDAStream().stream();
+    const int rc = launch(*reinterpret_cast<const unit_conv_plan *>(plan_addr), st);
+    if (rc) return PyLong_FromLong(rc);
+    keep(self, plan_addr, args[1], reinterpret_cast<void *>(ws_addr), c_out, op, args + 5, nargs - 5, st);
     Py_RETURN_NONE;
   } catch (...) {
     return raise_in_python();
@@ -352,7 +357,7 @@ void launcher_dealloc(Launcher *self) {
 
 PyMethodDef launcher_methods[] = {
     {"call", (PyCFunction)(void (*)())launcher_call, METH_FASTCALL, "call(op, data, bias, residual, out, options...)"},
-    {"add", (PyCFunction)(void (*)())launcher_add, METH_FASTCALL, "add(plan, result, workspace, c_out, op, data, bias, residual, out, options...)"},
+    {"run", (PyCFunction)(void (*)())launcher_run, METH_FASTCALL, "run(plan, result, workspace, c_out, op, data, bias, residual, out, options...)"},
     {"add_stream", (PyCFunction)launcher_add_stream, METH_O, "the packed weights are ready on this stream"},
     {nullptr, nullptr, 0, nullptr}};
 PyTypeObject LauncherType = {PyVarObject_HEAD_INIT(nullptr, 0)};

@@ -105,10 +105,12 @@ class PackedWeights:
         self._ready = torch.cuda.Event()
         self._ready.record()
         self._synced = {_stream()}
-        # calls of known geometry run through the launcher, without the Python checks (csrc/host_ext.cpp)
-        self._launcher = _lib.host().Launcher(buf.device.index)
-        self._launcher.add_stream(_stream())
-        self._call = self._launcher.call
+        self._launcher = None   # made by the first call with these weights
+
+    @staticmethod
+    def _call(*call):
+        """Calls of known geometry: replaced by the launcher's (csrc/host_ext.cpp), which does without the Python checks."""
+        return None
 
     def sync_to_current_stream(self) -> None:
         """Make the current stream wait for the pack kernel, once per stream.  (Not while the stream
@@ -119,11 +121,19 @@ class PackedWeights:
             return
         torch.cuda.current_stream().wait_event(self._ready)
         self._synced.add(st)
-        self._launcher.add_stream(st)
+        if self._launcher is not None:
+            self._launcher.add_stream(st)
 
-    def _keep(self, plan: _CPlan, result: torch.Tensor, ws: Optional[torch.Tensor], c_out: int, *call) -> None:
-        """Hands the launcher the plan just made for this call (``call``: the arguments ``_call`` was tried with)."""
-        self._launcher.add(ctypes.addressof(plan), result, 0 if ws is None else ws.data_ptr(), c_out, *call)
+    def _run(self, plan: _CPlan, result: torch.Tensor, ws: Optional[torch.Tensor], c_out: int, *call) -> None:
+        """Launches the plan made for this call and keeps it (``call``: the arguments ``_call`` was tried with)."""
+        if self._launcher is None:
+            launcher = _lib.host().Launcher(self.buf.device.index)
+            for st in self._synced:
+                launcher.add_stream(st)
+            self._launcher, self._call = launcher, launcher.call
+        r = self._launcher.run(ctypes.addressof(plan), result, 0 if ws is None else ws.data_ptr(), c_out, *call)
+        if r is not None:
+            check(r, 'unit_conv2d_run')
 
     @property
     def nbytes(self) -> int:
@@ -382,12 +392,15 @@ def conv2d_NCHWc_int8(data: torch.Tensor, kernel, stride: IntPair = 1, padding: 
     if n > 0:
         x, pw = tensors[0], tensors[1]
         with torch.cuda.device(x.device):
-            plan = _CPlan()
-            check(L.unit_conv2d_plan_int8(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
-                                          ws_bytes, ctypes.byref(plan)), 'unit_conv2d_plan_int8')
-            check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
-            pw._keep(plan, out_t, ws, d.c_out, _CONV2D, data, bias, residual, out, stride, padding, dilation, out_layout, out_dtype,
-                     requant_shift, mul)
+            if pw is kernel:
+                plan = _CPlan()
+                check(L.unit_conv2d_plan_int8(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
+                                              ws_bytes, ctypes.byref(plan)), 'unit_conv2d_plan_int8')
+                pw._run(plan, out_t, ws, d.c_out, _CONV2D, data, bias, residual, out, stride, padding, dilation, out_layout, out_dtype,
+                        requant_shift, mul)
+            else:   # (weights that the call packed itself: their next call comes through here again)
+                check(L.unit_conv2d_int8_nchwc(ctypes.byref(d), _ptr(x), _ptr(pw.buf), ctypes.byref(epi), _ptr(out_t), _ptr(ws),
+                                               ws_bytes, _stream()), 'unit_conv2d_int8_nchwc')
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -537,12 +550,14 @@ def dense_dotprod(data: torch.Tensor, weight, bias: Optional[torch.Tensor] = Non
             out_t = out
             if tuple(out_t.shape) != (m, n) or out_t.dtype != torch.int32 or not out_t.is_cuda or not out_t.is_contiguous():
                 raise ValueError('out must be a contiguous CUDA int32 [M][N] tensor')
-        if m > 0:
+        if m > 0 and pw is weight:
             plan = _CPlan()
             check(L.unit_dense_plan_u8s8s32(m, n, k, _ptr(data), k, _ptr(pw.buf), _ptr(out_t), n, ctypes.byref(plan)),
                   'unit_dense_plan_u8s8s32')
-            check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
-            pw._keep(plan, out_t, None, n, _DENSE, data, None, None, out)
+            pw._run(plan, out_t, None, n, _DENSE, data, None, None, out)
+        elif m > 0:
+            check(L.unit_dense_u8s8s32(m, n, k, _ptr(data), k, _ptr(pw.buf), _ptr(out_t), n, _stream()),
+                  'unit_dense_u8s8s32')
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -669,11 +684,14 @@ def conv2d_NCHW16c_OHWI16o(a: torch.Tensor, b, stride_h: int = 1, stride_w: int 
                 raise ValueError(f'out must be a contiguous CUDA float32 tensor of shape {oshape}')
         if n == 0:
             return out_t.cpu() if (host and out is None) else out_t
-        plan = _CPlan()
-        check(L.unit_conv2d_plan_f16f32(ctypes.byref(d), _ptr(a), _ptr(pw.buf), _ptr(out_t), ctypes.byref(plan)),
-              'unit_conv2d_plan_f16f32')
-        check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
-        pw._keep(plan, out_t, None, c_out, _CONV_F16, *call)
+        if pw is b:
+            plan = _CPlan()
+            check(L.unit_conv2d_plan_f16f32(ctypes.byref(d), _ptr(a), _ptr(pw.buf), _ptr(out_t), ctypes.byref(plan)),
+                  'unit_conv2d_plan_f16f32')
+            pw._run(plan, out_t, None, c_out, _CONV_F16, *call)
+        else:
+            check(L.unit_conv2d_f16f32_nchw16c(ctypes.byref(d), _ptr(a), _ptr(pw.buf), _ptr(out_t), _stream()),
+                  'unit_conv2d_f16f32_nchw16c')
     return out_t.cpu() if (host and out is None) else out_t
 
 
@@ -720,12 +738,14 @@ def gemm_f16f32(a: torch.Tensor, b, *, out: Optional[torch.Tensor] = None) -> to
             out_t = out
             if tuple(out_t.shape) != (m, n) or out_t.dtype != torch.float32 or not out_t.is_cuda or not out_t.is_contiguous():
                 raise ValueError('out must be a contiguous CUDA float32 [M][N] tensor')
-        if m > 0:
+        if m > 0 and pw is b:
             plan = _CPlan()
             check(L.unit_gemm_plan_f16f32(m, n, k, _ptr(a), 2 * k, _ptr(pw.buf), _ptr(out_t), n, ctypes.byref(plan)),
                   'unit_gemm_plan_f16f32')
-            check(L.unit_conv2d_run(ctypes.byref(plan), _stream()), 'unit_conv2d_run')
-            pw._keep(plan, out_t, None, n, _GEMM, a, None, None, out)
+            pw._run(plan, out_t, None, n, _GEMM, a, None, None, out)
+        elif m > 0:
+            check(L.unit_gemm_f16f32(m, n, k, _ptr(a), 2 * k, _ptr(pw.buf), _ptr(out_t), n, _stream()),
+                  'unit_gemm_f16f32')
     return out_t.cpu() if (host and out is None) else out_t
 
 
