@@ -163,6 +163,26 @@ def test_narrow_tiles_conv(U, n, c, h, w, co, k, s):
         assert np.array_equal(got.cpu().numpy(), want), opt
 
 
+@pytest.mark.parametrize('m,n,k', [(128, 3072, 768), (4096, 1024, 512)])   # narrow tiles, whole column blocks
+def test_trace_marks_the_weight_copies(U, m, n, k):
+    from unit_b200 import _lib
+    L = _lib.lib()
+    a = torch.randint(0, 256, (m, k), dtype=torch.uint8, device='cuda')
+    pw = U.pack_dense_weights_int8(torch.randint(-128, 128, (n // 16, k // 4, 16, 4), dtype=torch.int8, device='cuda'))
+    U.dense_dotprod(a, pw)
+    trace = torch.zeros((4, 16), dtype=torch.int64, device='cuda')
+    torch.cuda.synchronize()
+    try:
+        assert L.unit_trace_attach(trace.data_ptr(), 4) == 0
+        U.dense_dotprod(a, pw)
+        torch.cuda.synchronize()
+    finally:
+        assert L.unit_trace_attach(None, 0) == 0
+    U.device_status()
+    row = trace[0].cpu().tolist()
+    assert row[2] > 0 and row[1] > 0, row
+
+
 @pytest.mark.parametrize('batch', [1, 16])
 def test_shared_plans_take_fewer_blocks_and_give_the_same_results(U, batch):
     """Launches that run beside others: SM time counts, so a small grid is cut less than for its own latency."""
