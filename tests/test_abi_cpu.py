@@ -122,3 +122,16 @@ def test_valid_call_without_a_device_reports_arch_not_a_crash(L):
     p = ctypes.c_void_p(addr)
     assert L.unit_conv2d_u8s8s32_nchwc(ctypes.byref(desc()), p, p, None, p, None, 0, None) == -5
     assert L.unit_dense_u8s8s32(8, 64, 64, p, 64, p, p, 64, None) == -5
+
+
+def test_the_host_extension_belongs_to_one_torch(L, monkeypatch):
+    """It is compiled against torch's C++ headers: under another torch its file is not taken, and is built anew."""
+    import importlib.metadata
+    import torch
+    from unit_b200 import _lib, build
+    assert torch.__version__ in os.path.basename(_lib.host().__file__) and _lib.host().__file__ == build.host_path()
+    monkeypatch.setattr(_lib, '_HOST', None)
+    monkeypatch.setattr(importlib.metadata, 'version', lambda name: '0.0.1')
+    assert '0.0.1' in build.host_path() and not build._newer(build.host_path(), build._HOST_DEPS)
+    with pytest.raises(ImportError):
+        _lib.host()

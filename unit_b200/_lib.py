@@ -6,6 +6,7 @@ operator fails with the reason.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 from . import build as _build
@@ -140,9 +141,12 @@ def host():
         return _HOST
     L = lib()
     import torch  # noqa: F401  (the extension links against torch's libraries, which this import loads)
-    if not os.path.exists(_build.HOST_PATH):
-        raise ImportError(f'unit_b200: {_build.HOST_PATH} is missing; build it with `python -m unit_b200.build`.')
-    from . import _host
+    path = _build.host_path()
+    if not os.path.exists(path):
+        raise ImportError(f'unit_b200: {path} is missing; build it with `python -m unit_b200.build`.')
+    spec = importlib.util.spec_from_file_location('unit_b200._host', path)
+    _host = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(_host)
     addr = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value  # noqa: E731
     _host.bind(addr(L.unit_conv2d_run), addr(L.unit_plan_rebind), addr(L.unit_pack_data_nchw_to_nchwc),
                addr(L.unit_unpack_data_nchwc_to_nchw))
