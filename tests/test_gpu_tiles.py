@@ -202,3 +202,12 @@ def test_shared_plans_take_fewer_blocks_and_give_the_same_results(U, batch):
     U.device_status()
     # per layer the time of a block grows as their number falls, but by less than the number does
     assert sum(shared.values()) < 0.9 * sum(alone.values()), (alone, shared)
+
+
+@pytest.mark.parametrize('n,c,h,co,k,small', [(1, 256, 14, 256, 1, True), (8, 256, 14, 256, 1, True), (8, 512, 7, 512, 3, True),
+                                              (64, 256, 14, 512, 1, False), (64, 64, 56, 64, 1, False)])
+def test_tuner_finds_the_grids_that_the_library_cuts_itself(U, n, c, h, co, k, small):
+    from unit_b200 import tune
+    x = torch.zeros((n, c // 16, h, h, 16), dtype=torch.uint8, device='cuda')
+    w = torch.zeros((co // 16, c // 16, k, k, 4, 16, 4), dtype=torch.int8, device='cuda')
+    assert tune.one_tile_per_sm(x, w, (1, 1), k // 2) == small

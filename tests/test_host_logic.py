@@ -185,3 +185,12 @@ def test_shape_corpus_parser_and_committed_corpus():
                       dict(n=1, c_in=256, h=14, w=14, c_out=512, kh=1, kw=1, stride_h=2, stride_w=2, count=1)]
     corpus = tile_table.load_corpus()
     assert len(corpus) >= 100 and all(s['c_in'] % 16 == 0 and s['c_out'] % 16 == 0 for s in corpus)
+
+
+def test_tuner_leaves_small_grids_to_the_library():
+    """Sizes of at most one tile per SM: column-block widths only, which hold for every input size."""
+    from unit_b200 import tune
+    shape = {'c_in': 64, 'c_out': 192, 'kh': 1, 'kw': 1, 'stride_h': 1, 'stride_w': 1, 'h': 14, 'w': 14}
+    assert all(c['mt'] == 0 and c['ksplit'] == 0 and c['bn'] for c in tune.candidates(shape, size_side=False))
+    assert tune.candidates(shape, weight_side=False, size_side=False) == []
+    assert {(c['mt'], c['ksplit']) for c in tune.candidates(shape)} == {(m, k) for m in (0, 1, 2) for k in (0, 1, 4, 8)}

@@ -7,7 +7,9 @@ convolution on the pre-padded sizes, at the logged batch 1 and at the batches gi
 library's own choice and the candidate overrides (column-block width, sub-tiles per tile, split-K
 limit) as CUDA-graph replays over several buffer sets, checks that every candidate reproduces the
 default's output bit for bit, and keeps an entry where a candidate beats the default by more than
-3 %.  The counterpart of the reference's tuning loops (apps/cpu/kernel/conv2d.py:56-75,
+3 %.  Sizes of at most one tile per SM get no sub-tile or split entries: there the library's own
+estimate picks the tile's width and the split together, and such an entry would switch it off or cap
+it.  The counterpart of the reference's tuning loops (apps/cpu/kernel/conv2d.py:56-75,
 python/tensorizer/tune.py).
 """
 from __future__ import annotations
@@ -19,7 +21,7 @@ import time
 
 import torch
 
-from . import ops, tile_table
+from . import _lib, ops, tile_table
 from .resnet50 import LAYERS
 
 
@@ -49,14 +51,27 @@ def _time_case(x_sets, w, stride, pad=0, reps=16):
     return a.elapsed_time(b) * 1e3 / (3 * reps * len(plans)), plans[0].out.clone()
 
 
-def candidates(shape, weight_side=True):
+def one_tile_per_sm(x, w, stride, pad) -> bool:
+    """Whether the library's own choice for this call is a grid of fewer tiles than SMs with single sub-tiles: the
+    grids whose tile width and split it estimates itself."""
+    L = _lib.lib()
+    plan = ops.conv2d_NCHWc_int8_plan(x, ops.pack_conv_weights_int8(w, stride, pad), stride=stride, padding=pad, out_dtype='uint8')
+    count = lambda: [L.unit_variant_launches(i) for i in range(L.unit_variant_count())]  # noqa: E731
+    before = count()
+    plan.run()
+    ran = [i for i, (a, b) in enumerate(zip(before, count())) if a != b]
+    single = all(b'MT=1' in L.unit_variant_name(i) for i in ran)
+    return single and plan.ctas < torch.cuda.get_device_properties(x.device).multi_processor_count
+
+
+def candidates(shape, weight_side=True, size_side=True):
     c_out = shape['c_out']
     bns = sorted({min(256, (c_out + 15) // 16 * 16), 128, 64} & set(range(16, 257, 16)))
     bns = [b for b in bns if b <= max(64, (c_out + 15) // 16 * 16)]
     out = []
     for bn in (bns if weight_side else []) + [0]:
-        for mt in (0, 1, 2):
-            for ks in (0, 1, 4, 8):
+        for mt in (0, 1, 2) if size_side else (0,):
+            for ks in (0, 1, 4, 8) if size_side else (0,):
                 if bn == 0 and mt == 0 and ks == 0:
                     continue
                 out.append({'bn': bn, 'kc': 0, 'mt': mt, 'ksplit': ks})
@@ -75,15 +90,17 @@ def tune_shape(shape, batch, sets=4, weight_side=True):
     tile_table.set_table([])
     pad = shape.get('pad', 0)
     base_us, base_out = _time_case(xs, w, stride, pad)
+    size_side = not one_tile_per_sm(xs[0], w, stride, pad)
     key = {k: shape[k] for k in ('c_in', 'c_out', 'kh', 'kw', 'stride_h', 'stride_w')}
     key['c_block'] = 16
     best = (base_us, None)
-    for cand in candidates(shape, weight_side):
+    for cand in candidates(shape, weight_side, size_side):
         # the weight-side fields (bn, kc) must sit in an entry for every input size; mt / ksplit in one for this size
         entries = []
         if cand['bn'] or cand['kc']:
             entries.append(dict(key, n=0, h=0, w=0, bn=cand['bn'], kc=cand['kc'], mt=0, ksplit=0))
-        entries.append(dict(key, n=batch, h=shape['h'], w=shape['w'], bn=0, kc=0, mt=cand['mt'], ksplit=cand['ksplit']))
+        if cand['mt'] or cand['ksplit']:
+            entries.append(dict(key, n=batch, h=shape['h'], w=shape['w'], bn=0, kc=0, mt=cand['mt'], ksplit=cand['ksplit']))
         try:
             tile_table.set_table(entries)
             us, out = _time_case(xs, w, stride, pad)
