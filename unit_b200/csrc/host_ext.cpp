@@ -148,7 +148,7 @@ bool push_out_dtype(Key &k, PyObject *o) {
   return true;
 }
 
-enum Op : int64_t { OP_CONV2D = 1, OP_CONV3D, OP_DENSE, OP_GEMM, OP_CONV_F16 };
+enum Op : int64_t { OP_CONV2D = 1, OP_DENSE, OP_GEMM, OP_CONV_F16 };
 
 // Positions of a call's arguments: every operator passes (data, bias, residual, out, options ...).
 constexpr Py_ssize_t kArgData = 0, kArgBias = 1, kArgResidual = 2, kArgOut = 3, kArgOptions = 4;
@@ -168,13 +168,6 @@ bool make_key(Key &k, int64_t op, PyObject *const *a, Py_ssize_t n, const at::Te
       if (!get_int_or_none(o[5], &v)) return false;
       k.push(v);
       if (!get_int(o[6], &v)) return false;
-      k.push(v);
-      return true;
-    case OP_CONV3D:  // stride, padding, out_dtype, requant_shift, mul
-      if (no != 5 || !push_tensor(k, x, 6) || !push_ints(k, o[0], 3) || !push_ints(k, o[1], 3) || !push_out_dtype(k, o[2])) return false;
-      if (!get_int_or_none(o[3], &v)) return false;
-      k.push(v);
-      if (!get_int(o[4], &v)) return false;
       k.push(v);
       return true;
     case OP_DENSE:

@@ -55,7 +55,7 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 # operator numbers of the launcher (csrc/host_ext.cpp)
-_CONV2D, _CONV3D, _DENSE, _GEMM, _CONV_F16 = 1, 2, 3, 4, 5
+_CONV2D, _DENSE, _GEMM, _CONV_F16 = 1, 2, 3, 4
 
 _TABLE_LOADED = False
 _HOST = None   # the bound extension, once a CUDA device and the library have been seen
