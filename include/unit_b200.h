@@ -262,7 +262,8 @@ int unit_conv2d_run(const unit_conv_plan *plan, void *stream);
 /* Points a plan at other buffers of the same shapes (the reference's built module is likewise called with
  * new arrays each time): tile selection and tensor map stay, only addresses change.  d_x is the activations
  * (or the A matrix), d_bias and d_residual are given exactly when the plan was made with them, d_workspace
- * when the plan uses scratch.  Not to be called while another thread uses the same plan. */
+ * when the plan uses scratch.  A refused call leaves the plan as it was.  Not to be called while another thread
+ * uses the same plan. */
 int unit_plan_rebind(unit_conv_plan *plan, const void *d_x, const int32_t *d_bias, const void *d_residual,
                      void *d_out, void *d_workspace);
 

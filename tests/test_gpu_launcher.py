@@ -191,3 +191,23 @@ def test_only_calls_with_packed_weights_pay_for_a_launcher(U):
         for t in raw + packed:
             assert torch.equal(t, raw[0])
     U.device_status()
+
+
+@pytest.mark.parametrize('case', CONV)
+def test_the_first_call_of_a_thread_runs_the_kept_plan(U, case, monkeypatch):
+    """A thread that has not used CUDA yet has no current context, which re-addressing a tensor map needs."""
+    import threading
+    g = gen(15)
+    pw, kw = conv_case(U, case, g)
+    xs = [u8(case['x'], g) for _ in range(4)]
+    want = [U.conv2d_NCHWc_int8_plan(x, pw, **kw).run() for x in xs]
+    U.conv2d_NCHWc_int8(xs[0], pw, **kw)
+    torch.cuda.synchronize()
+    calls, got = Calls(monkeypatch), {}
+    for i, x in enumerate(xs):
+        t = threading.Thread(target=lambda: got.update({i: U.conv2d_NCHWc_int8(x, pw, **kw)}))
+        t.start()
+        t.join()
+        assert torch.equal(got[i], want[i])
+    assert calls.n == 0
+    U.device_status()

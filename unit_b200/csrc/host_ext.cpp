@@ -248,11 +248,7 @@ PyObject *launcher_call(Launcher *self, PyObject *const *args, Py_ssize_t nargs)
       p.out = out.data_ptr();
     }
     if (!(e->at == p)) {
-      const int rc = g_rebind(&e->plan, p.x, static_cast<const int32_t *>(p.bias), p.residual, p.out, p.workspace);
-      if (rc) {
-        if (rc == UNIT_ERR_LAUNCH) e->key.n = 0;  // the plan is spent: its entry never matches again
-        Py_RETURN_NONE;
-      }
+      if (g_rebind(&e->plan, p.x, static_cast<const int32_t *>(p.bias), p.residual, p.out, p.workspace)) Py_RETURN_NONE;
       e->at = p;
     }
     const int rc = launch(e->plan, st);

@@ -1867,31 +1867,30 @@ int unit_plan_rebind(unit_conv_plan *plan, const void *x, const int32_t *bias, c
   IgemmParams &p = pl->p;
   // what the plan was made with or without stays so: the kernel variant and the bias step depend on it
   if ((p.bias != nullptr) != (bias != nullptr) || (p.residual != nullptr) != (residual != nullptr)) return UNIT_ERR_SHAPE;
-  const void *base = nullptr, *old_base = nullptr;
+  if (pl->fold_n > 0 && !workspace) return UNIT_ERR_NULL;
+  const void *base = pl->fold_n > 0 ? workspace : x, *old_base = pl->fold_n > 0 ? pl->fold_dst : p.a;
+  if (pl->map_base != 0 && base != old_base) {
+    alignas(64) CUtensorMap map;
+    memcpy(&map, pl->map, sizeof(map));
+    static const auto replace = driver_fn<CUresult (*)(CUtensorMap *, void *)>("cuTensorMapReplaceAddress");
+    if (!replace) return UNIT_ERR_LAUNCH;
+    if (replace(&map, const_cast<void *>(base)) != CUDA_SUCCESS) {
+      // a thread without a current context (this is its first use of CUDA): give it the device's and try again
+      int dev = 0;
+      if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || replace(&map, const_cast<void *>(base)) != CUDA_SUCCESS)
+        return UNIT_ERR_LAUNCH;
+    }
+    memcpy(pl->map, &map, sizeof(map));
+  }
+  // (nothing can fail from here on: a refused call leaves the plan as it was)
   if (pl->fold_n > 0) {
-    if (!workspace) return UNIT_ERR_NULL;
-    base = workspace;
-    old_base = pl->fold_dst;
     pl->fold_src = x;
     pl->fold_dst = workspace;
-  } else {
-    base = x;
-    old_base = p.a;
   }
   p.a = static_cast<const uint8_t *>(base);
   p.bias = bias;
   p.residual = static_cast<const uint8_t *>(residual);
   p.out = out;
-  if (pl->map_base != 0 && base != old_base) {
-    alignas(64) CUtensorMap map;
-    memcpy(&map, pl->map, sizeof(map));
-    static const auto replace = driver_fn<CUresult (*)(CUtensorMap *, void *)>("cuTensorMapReplaceAddress");
-    if (!replace || replace(&map, const_cast<void *>(base)) != CUDA_SUCCESS) {
-      pl->magic = 0;   // half rebound: unusable
-      return UNIT_ERR_LAUNCH;
-    }
-    memcpy(pl->map, &map, sizeof(map));
-  }
   return UNIT_OK;
 }
 
