@@ -211,3 +211,39 @@ def test_the_first_call_of_a_thread_runs_the_kept_plan(U, case, monkeypatch):
         assert torch.equal(got[i], want[i])
     assert calls.n == 0
     U.device_status()
+
+
+def test_a_stream_that_syncs_while_the_launcher_is_made(U, monkeypatch):
+    """Two threads make their first calls with the same weights at once: the launcher knows both streams."""
+    import threading
+    g = gen(16)
+    pw, kw = conv_case(U, CONV[0], g)
+    x = u8(CONV[0]['x'], g)
+    want = U.conv2d_NCHWc_int8_plan(x, pw, **kw).run()
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    calls = Calls(monkeypatch)
+
+    def on_other():
+        with torch.cuda.stream(other):
+            assert torch.equal(U.conv2d_NCHWc_int8(x, pw, **kw), want)
+
+    class Streams(set):
+        thread = None
+
+        def __iter__(self):     # (the launcher is being told the streams: the other thread's first call comes now)
+            known = list(set.__iter__(self))
+            if Streams.thread is None:
+                Streams.thread = threading.Thread(target=on_other)
+                Streams.thread.start()
+                Streams.thread.join(0.5)
+            return iter(known)
+
+    pw._synced = Streams(pw._synced)
+    U.conv2d_NCHWc_int8(x, pw, **kw)
+    Streams.thread.join()
+    n = calls.n
+    for _ in range(3):
+        on_other()
+    assert n == 2 and calls.n == n
+    U.device_status()

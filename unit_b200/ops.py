@@ -20,6 +20,7 @@ Reference counterparts (paths inside were/UNIT):
 from __future__ import annotations
 
 import ctypes
+import threading
 import weakref
 from typing import Optional, Sequence, Tuple, Union
 
@@ -94,6 +95,9 @@ def launch_count() -> int:
 # --------------------------------------------------------------------------
 # packed weights
 # --------------------------------------------------------------------------
+_LAUNCHER_LOCK = threading.Lock()
+
+
 class PackedWeights:
     """Tensor-core-ready copy of one weight tensor (device buffer + the geometry it was packed for)."""
 
@@ -120,17 +124,20 @@ class PackedWeights:
         if st in self._synced or torch.cuda.is_current_stream_capturing():
             return
         torch.cuda.current_stream().wait_event(self._ready)
-        self._synced.add(st)
-        if self._launcher is not None:
-            self._launcher.add_stream(st)
+        with _LAUNCHER_LOCK:
+            self._synced.add(st)
+            if self._launcher is not None:
+                self._launcher.add_stream(st)
 
     def _run(self, plan: _CPlan, result: torch.Tensor, ws: Optional[torch.Tensor], c_out: int, *call) -> None:
         """Launches the plan made for this call and keeps it (``call``: the arguments ``_call`` was tried with)."""
         if self._launcher is None:
-            launcher = _lib.host().Launcher(self.buf.device.index)
-            for st in self._synced:
-                launcher.add_stream(st)
-            self._launcher, self._call = launcher, launcher.call
+            with _LAUNCHER_LOCK:   # (threads may make their first calls at once: one launcher, which knows all their streams)
+                if self._launcher is None:
+                    launcher = _lib.host().Launcher(self.buf.device.index)
+                    for st in self._synced:
+                        launcher.add_stream(st)
+                    self._launcher, self._call = launcher, launcher.call
         r = self._launcher.run(ctypes.addressof(plan), result, 0 if ws is None else ws.data_ptr(), c_out, *call)
         if r is not None:
             check(r, 'unit_conv2d_run')
