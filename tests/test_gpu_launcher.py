@@ -247,3 +247,91 @@ def test_a_stream_that_syncs_while_the_launcher_is_made(U, monkeypatch):
         on_other()
     assert n == 2 and calls.n == n
     U.device_status()
+
+
+@pytest.mark.parametrize('case', CONV)
+def test_threads_share_packed_weights(U, case, monkeypatch):
+    """Each on its own stream with its own buffers, from the first call on; afterwards all of them run kept plans."""
+    import threading
+    g = gen(11)
+    xs = [u8(case['x'], g) for _ in range(4)]
+    calls = Calls(monkeypatch)
+    for round_ in range(4):
+        pw, kw = conv_case(U, case, g)
+        want = [U.conv2d_NCHWc_int8_plan(x, pw, **kw).run() for x in xs]
+        torch.cuda.synchronize()
+        barrier, errors, streams = threading.Barrier(4), [], [torch.cuda.Stream() for _ in range(4)]
+
+        def work(i, reps):
+            try:
+                with torch.cuda.stream(streams[i]):
+                    barrier.wait()
+                    for _ in range(reps):
+                        assert torch.equal(U.conv2d_NCHWc_int8(xs[i], pw, **kw), want[i])
+            except Exception as e:   # noqa: BLE001  (a thread's failure is the test's)
+                errors.append(e)
+
+        for reps in (3, 20):
+            n = calls.n
+            threads = [threading.Thread(target=work, args=(i, reps)) for i in range(4)]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            assert not errors, errors
+        assert calls.n == n     # the second time no call needed the checks
+    U.device_status()
+
+
+def test_calls_of_a_known_geometry_are_captured(U):
+    g = gen(12)
+    for case in CONV:
+        pw, kw = conv_case(U, case, g)
+        x = u8(case['x'], g)
+        out = torch.empty_like(U.conv2d_NCHWc_int8(x, pw, **kw))
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            U.conv2d_NCHWc_int8(x, pw, **kw)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            inner = U.conv2d_NCHWc_int8(x, pw, **kw)
+            U.conv2d_NCHWc_int8(x, pw, out=out, **kw)
+        for _ in range(2):
+            x.copy_(u8(case['x'], g))
+            graph.replay()
+            want = U.conv2d_NCHWc_int8_plan(x, pw, **kw).run()
+            assert torch.equal(inner, want) and torch.equal(out, want)
+    U.device_status()
+
+
+def test_more_geometries_than_are_kept(U, monkeypatch):
+    g = gen(13)
+    pw, _ = conv_case(U, dict(w=(4, 4, 3, 3, 4, 16, 4), stride=1, padding=1), g)
+    calls = Calls(monkeypatch)
+    for n_seen, h in enumerate(list(range(5, 75)) + [5, 74]):
+        x = u8((1, 4, h, 7, 16), g)
+        for _ in range(2):
+            assert torch.equal(U.conv2d_NCHWc_int8(x, pw, padding=1), U.conv2d_NCHWc_int8_plan(x, pw, padding=1).run())
+    # per geometry one call with the checks (the other prepared launch is the reference); the oldest one was evicted
+    assert calls.n == 72 * 2 + 71
+    U.device_status()
+
+
+def test_a_new_tile_table_plans_anew(U, monkeypatch):
+    from unit_b200 import tile_table
+    g = gen(14)
+    pw, kw = conv_case(U, dict(w=(4, 4, 3, 3, 4, 16, 4), stride=1, padding=1), g)
+    x = u8((2, 4, 28, 28, 16), g)
+    want = U.conv2d_NCHWc_int8(x, pw, **kw)
+    calls = Calls(monkeypatch)
+    try:
+        tile_table.set_table([dict(c_in=64, c_out=64, kh=3, kw=3, stride_h=1, stride_w=1, n=2, h=28, w=28, mt=1, ksplit=1)])
+        for _ in range(2):
+            assert torch.equal(U.conv2d_NCHWc_int8(x, pw, **kw), want)
+        assert calls.n == 1
+    finally:
+        tile_table.load_default_table()
+    assert torch.equal(U.conv2d_NCHWc_int8(x, pw, **kw), want) and calls.n == 2
+    U.device_status()

@@ -306,7 +306,7 @@ def test_resnet50_sweep_config3(U, oracle, batch):
 @pytest.mark.parametrize('m,n,k,t', [
     (1, 16, 16, 16), (128, 3072, 768, 128), (100, 128, 128, 128), (300, 512, 1024, 128), (129, 48, 80, 16),
     (1024, 1024, 1024, 16),
-    # swizzled A rows (K a multiple of 128 bytes) with ragged M and N, and K just off that grid (column copies)
+    # ragged M and N, K a multiple of 128 bytes and off that grid: swizzled rows from 128 KB on, the gather below
     (257, 272, 384, 16), (5, 16, 128, 16), (700, 528, 2048, 16), (130, 64, 144, 16),
 ])
 def test_dense_int8_bit_exact(U, oracle, m, n, k, t):

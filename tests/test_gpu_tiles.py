@@ -83,6 +83,36 @@ def test_gemm_column_copies_after_another_kernel(U, m, n, k):
         gemm_case(U, m, n, k)
 
 
+# the same form on bytes: every reduction below 128 bytes with a matrix of 128 KB and more
+@pytest.mark.parametrize('m,n,k', [(8200, 64, 16), (40007, 64, 16), (4100, 272, 32), (2800, 48, 48), (40007, 128, 64), (1700, 528, 80),
+                                   (1400, 16, 96), (1200, 64, 112)])
+def test_dense_column_copies(U, m, n, k):
+    from unit_b200 import _lib
+    columns = (k // 16 + 1) & ~1
+    per_row = _lib.lib().unit_packed_weights_bytes_dense_i8(n, k) // 16
+    assert m * k >= 131072 and (per_row < n * 8 if k < 112 else per_row % (n * columns) == 0)   # (112: a stage of 8 columns)
+    names = dense_case(U, m, n, k)
+    assert all('A_DENSE_TMA' in v for v in names), names
+
+
+# rows further apart than they are long, reductions that end inside a 128-byte stage and inside a K step
+@pytest.mark.parametrize('m,n,k,gap', [(700, 272, 1040, 48), (2050, 64, 208, 16), (300, 528, 1104, 1024), (9000, 48, 80, 32)])
+def test_dense_rows_with_a_gap(U, m, n, k, gap):
+    import ctypes
+    from unit_b200 import _lib
+    L = _lib.lib()
+    rng = np.random.default_rng(m + k)
+    a = rng.integers(0, 256, (m, k + gap), dtype=np.uint8)     # (what lies in the gap must not enter the sums)
+    b = rng.integers(-128, 128, (n, k), dtype=np.int8)
+    ad, pw = dev(a), U.pack_dense_weights_int8(dev(no.pack_dense_weights(b, 16)))
+    got = torch.full((m, n + 16), 7, dtype=torch.int32, device='cuda')
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert L.unit_dense_u8s8s32(m, n, k, ad.data_ptr(), k + gap, pw.buf.data_ptr(), got.data_ptr(), n + 16, st) == 0
+    U.device_status()
+    want = (ad[:, :k].double() @ dev(b).double().t()).to(torch.int32)
+    assert torch.equal(got[:, :n], want) and bool((got[:, n:] == 7).all())
+
+
 # (batch, chunks, depth, h, w, c_out, kernel, padding): one and two sub-tiles, padding in no and in every dimension,
 # kernels that are flat in one dimension, slices smaller than a tile, a column block that is not full
 @pytest.mark.parametrize('n,c,d,h,w,co,k,p', [
@@ -109,9 +139,37 @@ def test_conv3d_windows_over_the_whole_batch(U, n, c, d, h, w, co, k, p):
     U.device_status()
 
 
-# every form of the final pack: the shorter one (8), a dot product that scales the residual (up to 15), plain adds
-# above; with one and two sub-tiles per tile, a ragged last column block and sums on both sides of the clamp
-@pytest.mark.parametrize('shift', [1, 7, 8, 9, 15, 16, 23])
+def test_conv3d_window_with_a_residual(U):
+    """Through the C ABI: the Python operator has no residual in three dimensions."""
+    import ctypes
+    from oracle import c_oracle
+    from unit_b200 import _lib
+    L = _lib.lib()
+    n, c, d, h, w, co = 3, 64, 14, 44, 44, 48
+    rng = np.random.default_rng(5)
+    x = rng.integers(0, 256, (n, c // 16, d, h, w, 16), dtype=np.uint8)
+    wt = rng.integers(-128, 128, (co // 16, c // 16, 3, 3, 3, 4, 16, 4), dtype=np.int8)
+    b = rng.integers(-2 ** 15, 2 ** 15, co, dtype=np.int32)
+    acc = c_oracle.conv3d_u8s8(x, wt, (1, 1, 1), (1, 1, 1), bias=b)
+    r = rng.integers(0, 256, acc.shape, dtype=np.uint8)
+    xd, bd, rd = dev(x), dev(b), dev(r)
+    pw = U.pack_conv3d_weights_int8(dev(wt), 1)
+    got = torch.empty(acc.shape, dtype=torch.uint8, device='cuda')
+    desc = _lib.Conv3dDesc(n, c, d, h, w, co, 3, 3, 3, 1, 1, 1, 1, 1, 1)
+    epi = _lib.Epilogue(bd.data_ptr(), 1, 10, 1, rd.data_ptr(), 0)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rc, names = launched(lambda: L.unit_conv3d_int8_ncdhwc(ctypes.byref(desc), xd.data_ptr(), pw.buf.data_ptr(), ctypes.byref(epi),
+                                                           got.data_ptr(), st))
+    assert rc == 0 and all('A_CONV_WIN, EPI_RES_NCHWC' in v for v in names), (rc, names)
+    U.device_status()
+    want = np.clip(((acc.astype(np.int64) + 512) >> 10) + r, 0, 255).astype(np.uint8)
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
+# every form of the final pack: the shorter one (8), any other while bias and rounding constant fit the bias step (18
+# at most), a dot product that scales the residual (up to 15); the general loop above those; with one and two sub-tiles
+# per tile, a ragged last column block and sums on both sides of the clamp
+@pytest.mark.parametrize('shift', [1, 7, 8, 9, 15, 16, 17, 18, 19, 20, 23])
 @pytest.mark.parametrize('n,c,h,co', [(9, 32, 23, 48), (32, 64, 28, 272)])
 def test_requantising_drains_at_every_shift(U, n, c, h, co, shift):
     from oracle import c_oracle

@@ -142,12 +142,12 @@ def test_fp16_conv_variants(U, oracle, case):
 
 
 DENSE_CASES = {
-    # (m, n, k): matrices of at least 128 KB arrive by tensor copies (128-byte-swizzled rows when K is a
-    # multiple of 128 bytes, 16-byte columns otherwise); smaller ones by the cp.async gather
+    # (m, n, k): matrices of at least 128 KB arrive by tensor copies (128-byte-swizzled rows, or 16-byte columns for
+    # reductions below one such row in both types); smaller ones by the cp.async gather
     'tma_sw128_mt1': ((10000, 64, 384), 'A_DENSE_TMA, EPI_RAW_ROWS, {}, MT=1'),
     # the reference's split-K GEMM shape (poc/tensorcore/gemm-prefetch.cu: 128 x 768 x 3072): three tiles, eight CTAs each
     'tma_splitk': ((128, 768, 3072), 'A_DENSE_TMA, EPI_RAW_ROWS, {}, MT=1, split-K'),
-    'tma_cols_mt1': ((2000, 64, 144), 'A_DENSE_TMA, EPI_RAW_ROWS, {}, MT=1'),
+    'tma_cols_mt1': ((5000, 64, 48), 'A_DENSE_TMA, EPI_RAW_ROWS, {}, MT=1'),
     'tma_mt2': ((20000, 16, 128), 'A_DENSE_TMA, EPI_RAW_ROWS, {}, MT=2'),
     'gather_mt1': ((129, 48, 80), 'A_DENSE, EPI_RAW_ROWS, {}, MT=1'),
 }

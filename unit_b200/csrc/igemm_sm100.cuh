@@ -18,8 +18,8 @@
 // are one 16-byte core-matrix row and consecutive pixels of an image row are
 // consecutive rows.  The A tile is filled by tensor copies (TMA): whole-row
 // boxes for stride 1, im2col-mode copies for other strides, column copies for
-// plain matrices; 16-byte cp.async gathers with zero fill remain as the path
-// for small tensors and NCHW4c without scratch.  Weights are repacked once on
+// plain matrices with rows below 128 bytes; 16-byte cp.async gathers with zero
+// fill remain as the path for small tensors and NCHW4c without scratch.  Weights are repacked once on
 // the device into ready-made [KC][BN][16 B] stage blocks and arrive with a
 // single bulk copy (cp.async.bulk, no tensor map, no multicast) per stage.
 //
@@ -657,7 +657,8 @@ __device__ __forceinline__ uint4 pack16_shift8(const uint32_t *t) {
                        pack_sat_u16((int32_t)t[4 * q + 3], (int32_t)t[4 * q + 2]), 0x7531);
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
-// The same for any other shift (1 .. 23): 16 more shifts per group.
+// The same for any other shift: 16 more shifts per group.  (Final accumulators hold the rounding constant 2^(shift-1)
+// in the bias step, whose digits end at 243967: shifts up to 18 come here.)
 __device__ __forceinline__ uint4 pack16_shift(const uint32_t *t, int shift) {
   uint32_t w[4];
 #pragma unroll
