@@ -51,3 +51,20 @@ def test_misaligned_tensors_and_no_writes_outside(hw, shift):
     assert torch.equal(back[shift:shift + size], src[shift:shift + size])
     for t, k, v in ((dst, blocked, 7), (back, size, 9)):
         assert bool((t[:shift] == v).all()) and bool((t[shift + k:] == v).all())
+
+
+def test_more_channel_blocks_than_one_launch_numbers():
+    """Above 2^30 channel blocks a transform goes in two halves.  (Four channels of one pixel: both layouts are the
+    same bytes.)"""
+    import unit_b200 as U
+    n = 2 ** 30 + 5
+    if torch.cuda.mem_get_info()[0] < 16 * 2 ** 30:
+        pytest.skip('needs 16 GB')
+    x = torch.empty((n, 4, 1, 1), dtype=torch.uint8, device='cuda')
+    x.view(-1).view(torch.int32).copy_(torch.arange(n, dtype=torch.int32, device='cuda'))
+    y = U.pack_data_nchwc(x, 4)
+    assert y.shape == (n, 1, 1, 1, 4) and torch.equal(y.view(-1).view(torch.int32), x.view(-1).view(torch.int32))
+    back = U.unpack_data_nchwc(y)
+    assert torch.equal(back.view(-1).view(torch.int32), x.view(-1).view(torch.int32))
+    del x, y, back
+    torch.cuda.empty_cache()
