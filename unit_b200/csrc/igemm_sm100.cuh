@@ -1212,9 +1212,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
       const uint32_t run = (uint32_t)p.bn * 16u;
       const size_t block_bytes = (size_t)p.kc * (size_t)p.b_row_bytes;
       uint32_t s = 0, ring_phase = 0;
-      uint32_t lt = 0;
       bool alive = true;
-      for (int tile = tile0; tile < total_tiles && alive; tile += tstep, ++lt) {
+      for (int tile = tile0; tile < total_tiles && alive; tile += tstep) {
         const int n_tile = tile - (int)fast_div((uint32_t)tile, p.div_n_tiles) * p.n_tiles;
         const int block = n_tile / p.b_sub;
         const uint8_t *src = p.b + ((size_t)block * p.k_stages + ks_begin) * block_bytes + (size_t)(n_tile - block * p.b_sub) * run +
@@ -1230,8 +1229,8 @@ __global__ void __launch_bounds__(kNumThreads, 1)
           if (lane < p.kc) bulk_copy_g2s(smem_base + s * stage_bytes + a_stage_bytes + (uint32_t)lane * run, src, run, bar);
           if (++s == (uint32_t)p.stages) { s = 0; ring_phase ^= 1u; }
         }
-        if (lane == 0) trace_mark(p, lt, 2);
       }
+      if (lane == 0) trace_mark(p, 0, 2);  // (such a grid has one tile per CTA)
     }
   } else if (warp == kMmaWarp || (MT == 2 && warp == kMmaWarp2)) {
     // ===================== MMA issuers =====================
